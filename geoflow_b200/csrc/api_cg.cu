@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "gf_common.cuh"
+#include "k_cg_cluster.cuh"
 #include "k_dss.cuh"
 #include "k_vec.cuh"
 #include "ops_launch.cuh"
@@ -67,20 +68,23 @@ enum {
 // ---- unique-node maps ----
 // rows(f) visits every unique node once, calling f(c, g) with its index c
 // and (box only) lattice coordinates g; each(c, g, f) calls f(m) for the
-// members m of the node in ascending local id; mult(c, g) is the count.
+// members m of the node in ascending local id.
 
 // Box lattice of order N-1.  rows() walks lattice rows (fixed gy, gz) by
-// block, so a node's coordinates come from the launch shape; rows_sum() walks
-// the flat lattice index with multiply-shift divisions by the lattice
-// widths (FastDiv); the order being a compile-time constant turns every %
-// and / by p into a multiply-shift.
+// block, so a node's coordinates come from the launch shape; rows_sum() takes
+// runs of P lattice points per thread; the order being a compile-time constant
+// turns every % and / by p into a multiply-shift.
 template <int N>
 struct MapBox {
-  static constexpr int P = N - 1;
+  static constexpr int P = N - 1, NPTS = N;
   int dim, ne[3], per[3], M[3];
-  FastDiv fd0, fd1;  // divisions by M[0], M[1]
+  RunWalk<P> rw;
+  FastDiv fe0, fe1;  // divisions by ne[0], ne[1]
   static MapBox make(const BoxLattice &L) {
     MapBox m;
+    m.rw = RunWalk<P>::make(L);
+    m.fe0 = FastDiv::make(L.ne[0]);
+    m.fe1 = FastDiv::make(L.dim > 2 ? L.ne[1] : 1);
     m.dim = L.dim;
     m.sorted = 1;
     for (int d = 0; d < 3; d++) {
@@ -89,8 +93,6 @@ struct MapBox {
       m.M[d] = (int)L.M[d];
       if (d < L.dim && L.per[d] && L.ne[d] == 1) m.sorted = 0;
     }
-    m.fd0 = FastDiv::make(m.M[0]);
-    m.fd1 = FastDiv::make(m.M[1]);
     return m;
   }
   template <class F>
@@ -188,13 +190,10 @@ struct MapBox {
     for (int i = 0; i < k; i++) f((int64_t)m[i]);
   }
   // f(c, s) for every lattice point c, s = sum of its element copies in
-  // ascending local id (added in TS).  One thread per lattice point in
-  // lattice order (grid-stride over the flat index): the point's
-  // coordinates from two multiply-shift divisions, its copies from scalar
-  // offsets (lattice_offsets), added in the (z, y, x) nesting, which is
-  // ascending element id when no periodic direction has a single element
-  // (otherwise the explicit sort of each()).  Lattice and element-local
-  // sizes are below 2^31 (checked when the problem is created).
+  // ascending local id (added in TS).  One thread per run of P points (RunWalk,
+  // lattice.cuh; grid-stride): ascending element id when no periodic direction
+  // has a single element (otherwise the explicit sort of each()).  Lattice and
+  // element-local sizes are below 2^31 (checked when the problem is created).
   template <typename TS, typename TV, class F>
   __device__ __forceinline__ void rows_sum(const TV *__restrict__ inE, F f) const {
     if (!sorted) {
@@ -205,63 +204,66 @@ struct MapBox {
       });
       return;
     }
-    constexpr int NN = N * N;
-    const bool d3 = dim > 2;
-    const int nn = d3 ? NN * N : NN;
-    const int sy = ne[0] * nn, sz = ne[0] * ne[1] * nn;
-    const int nL = M[0] * M[1] * (d3 ? M[2] : 1);
-    const int stride = gridDim.x * blockDim.x;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nL;
-         c = (c < nL - stride) ? c + stride : nL) {
-      const int row = fd0.div(c), g0 = c - row * M[0];
-      const int g2 = fd1.div(row), g1 = row - g2 * M[1];
-      int ox0, ox1, oy0, oy1, oz0 = 0, oz1 = 0;
-      const int nx = lattice_offsets<P>(g0, ne[0], per[0], nn, 1, ox0, ox1);
-      const int ny = lattice_offsets<P>(g1, ne[1], per[1], sy, N, oy0, oy1);
-      const int nz = d3 ? lattice_offsets<P>(g2, ne[2], per[2], sz, NN, oz0, oz1) : 1;
-      TS s = TS(0);
+    runs([&](const LatRun &k) {
+      TS s[P] = {};
+      rw.first(k, [&](int r, int m) { s[r] = (TS)inE[m]; });
 #pragma unroll
-      for (int az = 0; az < 2; az++) {
-        if (az >= nz) break;
-        const int oz = az ? oz1 : oz0;
+      for (int r = 0; r < P; r++) s[r] = __fadd_rn_t(TS(0), s[r]);
+      rw.rest(k, [&](int r, int m) { s[r] = __fadd_rn_t(s[r], (TS)inE[m]); });
 #pragma unroll
-        for (int ay = 0; ay < 2; ay++) {
-          if (ay >= ny) break;
-          const int o = oz + (ay ? oy1 : oy0);
-          s = __fadd_rn_t(s, (TS)inE[o + ox0]);
-          if (nx > 1) s = __fadd_rn_t(s, (TS)inE[o + ox1]);
-        }
-      }
-      f((int64_t)c, s);
+      for (int r = 0; r < P; r++)
+        if (r == 0 || k.body) f((int64_t)(k.c + r * rw.ls), s[r]);
+    });
+  }
+  // g(k) for every run (or single point) of the lattice
+  template <class G>
+  __device__ __forceinline__ void runs(G g) const {
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    if (rw.one) {
+      for (int t = t0; t < rw.npts; t = (t < rw.npts - stride) ? t + stride : rw.npts)
+        g(rw.point(t));
+    } else {
+      for (int t = t0; t < rw.n; t = (t < rw.n - stride) ? t + stride : rw.n) g(rw.run(t));
     }
   }
-  __device__ __forceinline__ double mult(int64_t, const int (&g)[3]) const {
-    int m = 1;
-    for (int d = 0; d < dim; d++) {
-      int ec[2], l[2];
-      m *= cands(d, g[d], ec, l);
+  // f(c, v), v = the first copy (smallest member) of lattice point c in inE
+  template <typename TV, class F>
+  __device__ __forceinline__ void pick(const TV *__restrict__ inE, F f) const {
+    if (!sorted) {
+      rows([&](int64_t c, const int(&g)[3]) {
+        bool first = true;
+        TV v = TV(0);
+        each(c, g, [&](int64_t m) {
+          if (first) v = inE[m];
+          first = false;
+        });
+        f(c, v);
+      });
+      return;
     }
-    return (double)m;
+    runs([&](const LatRun &k) {
+      rw.first(k, [&](int r, int m) { f((int64_t)(k.c + r * rw.ls), inE[m]); });
+    });
   }
-  __device__ __forceinline__ int64_t lof(int64_t i) const {  // E index -> lattice index
-    constexpr int NN = N * N;
-    const int64_t nn = dim > 2 ? (int64_t)NN * N : NN;
-    const int64_t e = i / nn;
-    const int a = (int)(i - e * nn);
-    const int c0 = (int)(e % ne[0]);
-    const int64_t r = e / ne[0];
-    const int c1 = (int)(r % ne[1]), c2 = dim > 2 ? (int)(r / ne[1]) : 0;
+  // E index -> lattice index (sizes below 2^31)
+  __device__ __forceinline__ int64_t lof(int64_t i) const {
+    constexpr unsigned NN = N * N;
+    const unsigned ui = (unsigned)i, e = dim > 2 ? ui / (NN * N) : ui / NN;
+    const unsigned a = ui - e * (dim > 2 ? NN * N : NN);
+    const int r = fe0.div((int)e), c0 = (int)e - r * ne[0];
+    const int c2 = dim > 2 ? fe1.div(r) : 0, c1 = r - c2 * ne[1];
     auto g1 = [&](int d, int ec, int l) {
       int gi = ec * P + l;
       return (per[d] && gi == M[d]) ? 0 : gi;
     };
-    int64_t idx = g1(0, c0, a % N) + (int64_t)M[0] * g1(1, c1, (a / N) % N);
-    if (dim > 2) idx += (int64_t)M[0] * M[1] * g1(2, c2, a / NN);
+    int idx = g1(0, c0, a % N) + M[0] * g1(1, c1, (a / N) % N);
+    if (dim > 2) idx += M[0] * M[1] * g1(2, c2, a / NN);
     return idx;
   }
 };
 
 struct MapCsr {
+  static constexpr int NPTS = 0;
   const int32_t *ptr, *mem, *ncls;
   int64_t nL;
   template <class F>
@@ -275,8 +277,11 @@ struct MapCsr {
   __device__ __forceinline__ void each(int64_t c, const int (&)[3], F f) const {
     for (int32_t k = ptr[c]; k < ptr[c + 1]; k++) f((int64_t)mem[k]);
   }
-  __device__ __forceinline__ double mult(int64_t c, const int (&)[3]) const {
-    return (double)(ptr[c + 1] - ptr[c]);
+  template <typename TV, class F>
+  __device__ __forceinline__ void pick(const TV *__restrict__ inE, F f) const {
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < nL;
+         c += (int64_t)gridDim.x * blockDim.x)
+      f(c, inE[mem[ptr[c]]]);
   }
   template <typename TS, typename TV, class F>
   __device__ __forceinline__ void rows_sum(const TV *__restrict__ inE, F f) const {
@@ -330,15 +335,7 @@ __global__ void k_assemble(int64_t nL, MAP map, const TI *__restrict__ inE, doub
 // x_L[c] = x_E[smallest member]  (x_E is duplicate-consistent)
 template <class MAP>
 __global__ void k_pick(int64_t nL, MAP map, const double *__restrict__ xE, double *__restrict__ xL) {
-  map.rows([&](int64_t c, const int(&g)[3]) {
-    bool first = true;
-    double v = 0.0;
-    map.each(c, g, [&](int64_t m) {
-      if (first) v = xE[m];
-      first = false;
-    });
-    xL[c] = v;
-  });
+  map.pick(xE, [&](int64_t c, double v) { xL[c] = v; });
 }
 
 // x_E = mask_E * x_L[class] + xb_E   (solve_impl (2) epilogue)
@@ -597,6 +594,48 @@ __global__ void k_wupdate(int64_t nL, T *__restrict__ w, const T *__restrict__ r
     const T rc = r[c];
     const T zc = dinv ? (T)dinv[c] * rc : rc;
     w[c] = beta * w[c] + T(1) * zc;
+  }
+}
+
+// K1 and W as kernel arguments
+struct ClBasis {
+  double K1[GF_MAXN * GF_MAXN], W[GF_MAXN];
+};
+
+// The whole FP64 iteration of a small 2-d box in one cluster (k_cg_cluster.cuh):
+// initial residual, GCG's stop rule on norm(b) (scal[S_BNORM]) and the scalar
+// block as k_resid (mode 0) and the iteration kernels leave it.
+template <int N>
+__global__ void __launch_bounds__(CL_THREADS, 1)
+    k_cg_cluster(const __grid_constant__ ClProblem b, const __grid_constant__ ClBasis B, double tol,
+                 double *hist, double *scal) {
+  __shared__ ClShared sh;
+  extern __shared__ __align__(16) double slab[];
+  cl_load_basis(sh, N, B.K1, B.W, b);
+  const double bnorm = scal[S_BNORM];
+  const int limit = (int)scal[S_MAXIT];
+  const double stop = (scal[S_REL] != 0.0 || bnorm >= 1.0) ? tol * bnorm : tol;
+  ClState st;
+  bool run = false;
+  cl_solve_any<N>(
+      b, sh, slab, st,
+      [&](ClState &s, double &rtol, int &maxit) {
+        rtol = stop;
+        maxit = limit;
+        s.rnorm = 10.0 * stop;  // GCG's loop runs at least once
+        s.bad = s.bad || !isfinite(bnorm);
+        run = !s.bad && limit > 0 && 10.0 * stop > stop;
+        return run;
+      },
+      hist);
+  if (cl_rank() == 0 && threadIdx.x == 0) {
+    scal[S_RES] = st.res;
+    scal[S_RTOL] = scal[S_OTOL] = stop;
+    scal[S_RNORM] = st.rnorm;
+    scal[S_RHO] = st.rho;
+    scal[S_ITER] = (double)st.iters;
+    scal[S_FLAG] = st.bad ? 1.0 : 0.0;
+    scal[S_DONE] = run ? 2.0 : 1.0;
   }
 }
 
@@ -1130,86 +1169,70 @@ __global__ void k_mg_start(int64_t nL, const double *__restrict__ r64, TM *__res
 enum { MG_STEP = 0, MG_RESID = 1, MG_START = 3, MG_FOLDB = 4 };
 enum { DP_NONE = 0, DP_X = 1, DP_D = 2 };
 
-// One thread per lattice point, in lattice order (grid-stride over the
-// flat index): the state vectors stream fully coalesced, and a warp's
-// copies of one element row are one 32-byte sector of qE.  The point's
-// coordinates come from two multiply-shift divisions, its copies from
-// scalar offsets (no local arrays), its state loads are issued before the
-// gather (one memory round trip per point), and the copies are added in the
-// (z, y, x) nesting of MapBox::rows_sum (ascending element id unless a
-// periodic direction has a single element).  Lattice and element-local
-// sizes are below 2^31 (checked when the problem is created).
-// (Measured on B200 against this form: element-ordered walks, lattice rows
-// mapped to power-of-two thread groups, several points per thread, z-column
-// walks and a lattice-row layout of qE were all slower.)
-template <int N, int MODE, bool DOTS, typename TM>
+// One thread per run of P lattice points (RunWalk, lattice.cuh; grid-stride):
+// the state vectors stream coalesced, P loads of each in flight per thread and
+// issued before the gather, and the index arithmetic is paid once per run; the
+// copies of a point are added in the (z, y, x) nesting (ascending element id
+// unless a periodic direction has a single element).  One thread per point
+// executed 133 instructions per point, most of them index arithmetic.
+// (ONE: a point per thread, RunWalk::one; in one kernel with the runs it cost them
+// registers, FP32 p = 7 step 60 -> 80 us.)
+template <int N, int MODE, bool DOTS, typename TM, bool ONE>
 __global__ void __launch_bounds__(RED_THREADS)
-    k_mg_pass_lat(MapBox<N> map, Weights wt,
+    k_mg_pass_lat(const RunWalk<N - 1> w, Weights wt,
                   const TM *__restrict__ qE, TM *__restrict__ b,
                   const TM *__restrict__ dinv, TM c1, TM c2, TM *__restrict__ res,
                   TM *__restrict__ d, TM *__restrict__ x, int dsrc, int wd, double *scal,
                   double *partials, unsigned int *counter) {
   __shared__ double sh[32];
   if (scal[S_DONE] != 0.0) return;
-  constexpr int P = N - 1, NN = N * N;
+  constexpr int P = N - 1;
   double rz = 0.0;
-  const bool d3 = map.dim > 2;
-  const int nn = d3 ? NN * N : NN;
-  const int ne0 = map.ne[0], ne1 = map.ne[1];
-  const int M0 = map.M[0], M1 = map.M[1];
-  const int nL = M0 * M1 * (d3 ? map.M[2] : 1);
-  const int sy = ne0 * nn, sz = ne0 * ne1 * nn;
-  const int stride = gridDim.x * blockDim.x;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nL;
-       c = (c < nL - stride) ? c + stride : nL) {
-    const bool keep = !wt.maskL || wt.maskL[c];
-    TM bc = 0, xo = 0, dv = 0, dpv = 0;
-    if (MODE == MG_STEP || MODE == MG_RESID) bc = b[c];
-    if (MODE == MG_STEP || MODE == MG_START) dv = dinv[c];
-    if (MODE == MG_STEP) {
-      xo = x[c];
-      if (dsrc == DP_D) dpv = d[c];
-    }
-    const int row = map.fd0.div(c), g0 = c - row * M0;
-    const int g2 = map.fd1.div(row), g1 = row - g2 * M1;
-    int ox0, ox1, oy0, oy1, oz0 = 0, oz1 = 0;
-    const int nx = lattice_offsets<P>(g0, ne0, map.per[0], nn, 1, ox0, ox1);
-    const int ny = lattice_offsets<P>(g1, ne1, map.per[1], sy, N, oy0, oy1);
-    const int nz = d3 ? lattice_offsets<P>(g2, map.ne[2], map.per[2], sz, NN, oz0, oz1) : 1;
-    TM s = 0;
+  auto pass = [&](const LatRun &k) {
+    TM s[P] = {}, bc[P] = {}, dv[P] = {}, xo[P] = {}, dp[P] = {};
+    bool keep[P];
 #pragma unroll
-    for (int az = 0; az < 2; az++) {
-      if (az >= nz) break;
-      const int oz = az ? oz1 : oz0;
-#pragma unroll
-      for (int ay = 0; ay < 2; ay++) {
-        if (ay >= ny) break;
-        const int o = oz + (ay ? oy1 : oy0);
-        s = mg_add(s, qE[o + ox0]);
-        if (nx > 1) s = mg_add(s, qE[o + ox1]);
+    for (int r = 0; r < P; r++) {
+      const int c = k.c + r * w.ls;
+      const bool on = r == 0 || k.body;
+      keep[r] = on && (!wt.maskL || wt.maskL[c]);
+      if (!on) continue;
+      if (MODE == MG_STEP || MODE == MG_RESID) bc[r] = b[c];
+      if (MODE == MG_STEP || MODE == MG_START) dv[r] = dinv[c];
+      if (MODE == MG_STEP) {
+        xo[r] = x[c];
+        if (dsrc == DP_D) dp[r] = d[c];
       }
     }
-    if (!keep) s = 0;
-    if (MODE == MG_FOLDB) {
-      b[c] = s;
-      continue;
+    w.first(k, [&](int r, int m) { s[r] = qE[m]; });
+    w.rest(k, [&](int r, int m) { s[r] = mg_add(s[r], qE[m]); });
+#pragma unroll
+    for (int r = 0; r < P; r++) {
+      if (r > 0 && !k.body) continue;
+      const int c = k.c + r * w.ls;
+      if (!keep[r]) s[r] = 0;
+      if (MODE == MG_FOLDB) {
+        b[c] = s[r];
+      } else if (MODE == MG_START) {
+        b[c] = s[r];
+        x[c] = c1 * (dv[r] * s[r]);
+      } else if (MODE == MG_RESID) {
+        res[c] = bc[r] - s[r];
+      } else {
+        const TM rc = bc[r] - s[r];
+        const TM dc = c1 * (dsrc == DP_X ? xo[r] : dp[r]) + c2 * (dv[r] * rc);
+        const TM xc = xo[r] + dc;
+        x[c] = xc;
+        if (wd) d[c] = dc;
+        if (DOTS) rz += (double)bc[r] * (double)xc;
+      }
     }
-    if (MODE == MG_START) {
-      b[c] = s;
-      x[c] = c1 * (dv * s);
-      continue;
-    }
-    const TM rc = bc - s;
-    if (MODE == MG_RESID) {
-      res[c] = rc;
-      continue;
-    }
-    const TM dp = dsrc == DP_X ? xo : dpv;
-    const TM dc = c1 * dp + c2 * (dv * rc);
-    const TM xc = xo + dc;
-    x[c] = xc;
-    if (wd) d[c] = dc;
-    if (DOTS) rz += (double)bc * (double)xc;
+  };
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  if (ONE) {
+    for (int t = t0; t < w.npts; t = (t < w.npts - stride) ? t + stride : w.npts) pass(w.point(t));
+  } else {
+    for (int t = t0; t < w.n; t = (t < w.n - stride) ? t + stride : w.n) pass(w.run(t));
   }
   if (!DOTS) return;
   rz = block_reduce<false>(rz, sh);
@@ -1513,6 +1536,57 @@ struct Solver {
     });
   }
 
+  // small 2-d affine boxes iterate inside one cluster (CL_NODES)
+  bool cluster_ok() {
+    if (MAP::NPTS == 0 || prob->dim != 2 || !prob->egeom_d || nL > CL_NODES) return false;
+    if constexpr (MAP::NPTS > 0)
+      if (ctx->cluster_size == 0)
+        ctx->cluster_size = cl_cluster_size(k_cg_cluster<MAP::NPTS>, CL_THREADS);
+    return cl_slab_bytes((int)prob->box.M[0], (int)prob->box.M[1], prob->box.p,
+                         ctx->cluster_size) <= CL_SLAB_MAX;
+  }
+  int iterate_cluster(const gf_cg_traits &tr, double p, double q, int use_mass, const double *bL,
+                      double *xL, double *rL, double *w, double *qL, const float *dinv,
+                      double *hist, int *iters) {
+    if constexpr (MAP::NPTS > 0) {
+      ClProblem b = cl_problem(prob->box);
+      b.egeom = prob->egeom_d;
+      b.mask = wt.maskL;
+      b.mult = wt.multL;
+      b.massL = wt.massL;
+      b.dinv32 = dinv;
+      b.b = bL;
+      b.x = xL;
+      b.r = rL;
+      b.w = w;
+      b.q = qL;
+      b.p = p;
+      b.qm = use_mass ? q : 0.0;
+      b.normtype = tr.normtype;
+      b.ntot = (double)nE;
+      b.ivol = 1.0 / prob->volume;
+      ClBasis B;
+      std::copy(prob->K1, prob->K1 + prob->n * prob->n, B.K1);
+      std::copy(prob->W, prob->W + prob->n, B.W);
+      b.uniform = prob->egeom_uniform;
+      auto kern = k_cg_cluster<MAP::NPTS>;
+      const size_t smem = cl_slab_bytes(b.M0, b.M1, prob->box.p, ctx->cluster_size);
+      set_smem(kern, smem);
+      if (ctx->cluster_size == CL_MAX)
+        GF_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      prob->launches++;
+      GF_CUDA(ctx, cl_launch(kern, 1, ctx->cluster_size, CL_THREADS, smem, st, b, B, tr.tol, hist, prob->scal_d));
+      GF_CUDA(ctx, cudaMemcpyAsync(prob->scal_h, prob->scal_d, sizeof(double) * S_COUNT,
+                                   cudaMemcpyDeviceToHost, st));
+      GF_CUDA(ctx, cudaStreamSynchronize(st));
+      *iters = (int)prob->scal_h[S_ITER];
+      if (prob->scal_h[S_FLAG] != 0.0)
+        return gf_fail(ctx, GF_ERR_NONFINITE, "CG breakdown: non-finite scalar at iteration %d",
+                       *iters);
+    }
+    return GF_OK;
+  }
+
   // Queues iterations in batches of check_every (enq(k) queues k of them)
   // and reads the device `done` flag one batch behind, so the GPU never
   // waits for the host; stops at `done` or after maxit iterations.
@@ -1624,9 +1698,13 @@ struct Solver {
       double *w = (double *)gf_work(prob, 4, sizeof(double) * nL);
       double *qL = (double *)gf_work(prob, 5, sizeof(double) * nL);
       if (!w || !qL) return gf_fail(ctx, GF_ERR_NOMEM, "CG work allocation failed");
-      rc = residual<double>(p, q, use_mass, bL, xL, qE, rL, rL, w, d32, 0, tr.tol);
-      if (rc) return gf_fail(ctx, rc, "residual failed");
-      rc = iterate<double>(tr, tr.maxit, p, q, use_mass, xL, rL, w, qL, qE, d32, hist, &total);
+      if (cluster_ok()) {
+        rc = iterate_cluster(tr, p, q, use_mass, bL, xL, rL, w, qL, d32, hist, &total);
+      } else {
+        rc = residual<double>(p, q, use_mass, bL, xL, qE, rL, rL, w, d32, 0, tr.tol);
+        if (rc) return gf_fail(ctx, rc, "residual failed");
+        rc = iterate<double>(tr, tr.maxit, p, q, use_mass, xL, rL, w, qL, qE, d32, hist, &total);
+      }
       if (rc) return rc;
       rn = prob->scal_h[S_RNORM];
       rc = (total >= tr.maxit && rn > tr.tol) ? GF_CG_NOCONVERGE : GF_OK;
@@ -1807,8 +1885,9 @@ struct MGLevel : MGLevelBase<TM> {
   }
   template <int MODE, bool DOTS>
   void run_pass(TM a1, TM a2, int dsrc, int wd, gf_problem *outer, cudaStream_t st) {
-    auto kern = k_mg_pass_lat<N, MODE, DOTS, TM>;
-    kern<<<S.rgrid(kern), RED_THREADS, 0, st>>>(S.map, S.wt, qE, b, dinv, a1, a2, res, d, x, dsrc,
+    auto kern = S.map.rw.one ? k_mg_pass_lat<N, MODE, DOTS, TM, true>
+                             : k_mg_pass_lat<N, MODE, DOTS, TM, false>;
+    kern<<<S.rgrid(kern), RED_THREADS, 0, st>>>(S.map.rw, S.wt, qE, b, dinv, a1, a2, res, d, x, dsrc,
                                                  wd, outer->scal_d, outer->partials,
                                                  outer->counter);
   }

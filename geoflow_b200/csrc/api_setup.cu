@@ -495,6 +495,9 @@ extern "C" int gf_problem_create(gf_ctx_t ctx, const gf_problem_desc *d, gf_prob
   std::vector<double> jac(N), X0(N);
   if (d->geom == GF_GEOM_AFFINE) {
     std::vector<double> eg(d->elem_geom, d->elem_geom + d->ne * (dim + 1));
+    p->egeom_uniform = true;
+    for (size_t i = dim + 1; i < eg.size(); i++)
+      if (eg[i] != eg[i - (dim + 1)]) p->egeom_uniform = false;
     p->egeom_d = upload(eg);
     p->egeom_f = upload(to_f32(eg));
     for (int64_t e = 0; e < d->ne; e++)

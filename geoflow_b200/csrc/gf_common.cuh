@@ -21,6 +21,7 @@ struct gf_context {
   int nprob = 0;                // live problems created on this context
   bool destroy_pending = false; // destroyed while problems were alive
   int sm_count = 148;
+  int cluster_size = 0;  // CTAs per cluster of the one-cluster solves; 0: not asked yet
   std::string last_error;
   std::string returned_error;  // storage for gf_ctx_last_error
 };
@@ -46,6 +47,7 @@ struct gf_problem {
   // device geometry (both precisions)
   double *egeom_d = nullptr;  // ne*(dim+1) (AFFINE)
   float *egeom_f = nullptr;
+  bool egeom_uniform = false;   // AFFINE: every element has the first one's values
   double *ngeom_d = nullptr;  // (dim+1)*nlocal (REGULAR; DEFORMED/EMBEDDED: 0 planes + Jac)
   float *ngeom_f = nullptr;
   // DEFORMED / EMBEDDED: full dXi/dX (dim*nxy planes), packed metric G_ij

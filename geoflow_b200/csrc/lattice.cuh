@@ -248,4 +248,133 @@ struct BoxWalk {
   }
 };
 
+// The same points as BoxWalk, one run of P points per thread: thread t takes the
+// points of one lattice line along the last direction (z in 3-d, y in 2-d)
+// that share an element layer, offsets r = 0 .. P-1 from the layer's lower face.
+// The copies along the other directions are found once per run; r = 0 has one
+// or two copies along the last direction, r > 0 has one.  Consecutive threads
+// take consecutive x, so a warp's accesses are those of the lattice order, with
+// P independent loads per thread in flight and the index arithmetic of one
+// point for P of them.  A layer past a non-periodic upper boundary holds r = 0
+// alone.
+//
+// Lattices of fewer than POINT_NODES points are walked point by point (point()):
+// their runs are too few to cover the latency of the loads.  RK pass of three
+// components, FP64, p = 7: 80 k points 21 us in runs, 8 by points; V-cycle solves
+// at 227 k points, p = 5: 1.73 ms in runs, 1.61 by points, at 614 k, p = 7: 2.20
+// and 2.28.
+constexpr int POINT_NODES = 1 << 18;
+
+struct LatRun {
+  int o[4];      // offsets of the copies (y, x): (0,0), (0,1), (1,0), (1,1)
+  int nx, ny, nz;
+  int zA, zB;    // last-direction offsets of r = 0
+  int z0;        // last-direction offset of the layer
+  bool body;     // r > 0 exists
+  int c;         // lattice index of r = 0
+};
+
+template <int P>
+struct RunWalk {
+  int dim, M0, M1, n, npts, ne0, ne1, neL, per0, per1, perL, es0, es1, esL;
+  int ns, ls;  // stride of r in the element and in the lattice
+  FastDiv f0, f1;
+  bool one;    // a point per thread: point(t), t < npts, in place of run(t), t < n
+  static RunWalk make(const BoxLattice &L) {
+    RunWalk w;
+    const int N = P + 1, d = L.dim - 1;
+    w.dim = L.dim;
+    w.M0 = (int)L.M[0];
+    w.M1 = L.dim > 2 ? (int)L.M[1] : 1;
+    w.ne0 = L.ne[0];
+    w.per0 = L.per[0];
+    w.ne1 = L.dim > 2 ? L.ne[1] : 1;
+    w.per1 = L.dim > 2 ? L.per[1] : 0;
+    w.neL = L.ne[d];
+    w.perL = L.per[d];
+    w.es0 = L.dim > 2 ? N * N * N : N * N;
+    w.es1 = L.ne[0] * w.es0;
+    w.esL = L.dim > 2 ? L.ne[1] * w.es1 : w.es1;
+    w.ns = L.dim > 2 ? N * N : N;
+    w.ls = w.M0 * w.M1;
+    w.n = w.M0 * w.M1 * (w.neL + (w.perL ? 0 : 1));
+    w.f0 = FastDiv::make(w.M0);
+    w.f1 = FastDiv::make(w.M1);
+    w.npts = w.M0 * w.M1 * (int)L.M[d];
+    w.one = w.npts < POINT_NODES;
+    return w;
+  }
+  __host__ __device__ __forceinline__ int threads() const { return one ? npts : n; }
+  // the lattice point t (x fastest) as a run of r = 0 alone
+  __host__ __device__ __forceinline__ LatRun point(int t) const {
+    const int row = f0.div(t), g0 = t - row * M0;
+    const int z = dim > 2 ? f1.div(row) : row, q = z / P, r = z - q * P;
+    LatRun k = run(g0, dim > 2 ? row - z * M1 : 0, q);
+    if (r) {
+      k.zA = k.z0 + r * ns;
+      k.nz = 1;
+      k.c += r * ls;
+    }
+    k.body = false;
+    return k;
+  }
+  // the run of flat index t (x fastest) and of coordinates (g0, g1), layer q (2-d:
+  // g1 = 0)
+  __host__ __device__ __forceinline__ LatRun run(int t) const {
+    const int row = f0.div(t), g0 = t - row * M0;
+    const int q = dim > 2 ? f1.div(row) : row;
+    return run(g0, dim > 2 ? row - q * M1 : 0, q);
+  }
+  __host__ __device__ __forceinline__ LatRun run(int g0, int g1, int q) const {
+    LatRun k;
+    int x0, x1, y0 = 0, y1 = 0;
+    const int q0 = g0 / P, q1 = g1 / P;
+    k.nx = lattice_offsets_qr(q0, g0 - q0 * P, P, ne0, per0, es0, 1, x0, x1);
+    k.ny = 1;
+    if (dim > 2) k.ny = lattice_offsets_qr(q1, g1 - q1 * P, P, ne1, per1, es1, P + 1, y0, y1);
+    k.nz = lattice_offsets_qr(q, 0, P, neL, perL, esL, ns, k.zA, k.zB);
+    k.o[0] = y0 + x0;
+    k.o[1] = y0 + x1;
+    k.o[2] = y1 + x0;
+    k.o[3] = y1 + x1;
+    k.z0 = q * esL;
+    k.body = q < neL;
+    k.c = g0 + M0 * (g1 + (dim > 2 ? M1 : 1) * q * P);
+    return k;
+  }
+  // f(r, offset) over the first copies, and over the others, per point in the
+  // order of BoxWalk (z, y, x)
+  template <class F>
+  __host__ __device__ __forceinline__ void first(const LatRun &k, F f) const {
+    f(0, k.o[0] + k.zA);
+    if (k.body) {
+#pragma unroll
+      for (int r = 1; r < P; r++) f(r, k.o[0] + k.z0 + r * ns);
+    }
+  }
+  template <class F>
+  __host__ __device__ __forceinline__ void rest(const LatRun &k, F f) const {
+    auto line = [&](int o) {
+      f(0, o + k.zA);
+      if (k.body) {
+#pragma unroll
+        for (int r = 1; r < P; r++) f(r, o + k.z0 + r * ns);
+      }
+    };
+    if (k.nx > 1) line(k.o[1]);
+    if (k.ny > 1) {
+      line(k.o[2]);
+      if (k.nx > 1) line(k.o[3]);
+    }
+    if (k.nz > 1) {
+      f(0, k.o[0] + k.zB);
+      if (k.nx > 1) f(0, k.o[1] + k.zB);
+      if (k.ny > 1) {
+        f(0, k.o[2] + k.zB);
+        if (k.nx > 1) f(0, k.o[3] + k.zB);
+      }
+    }
+  }
+};
+
 }  // namespace gfk

@@ -52,6 +52,49 @@ static void check_fastdiv() {
   }
 }
 
+// RunWalk: every point once, its copies in BoxWalk's order
+template <int P>
+static void check_runs(const BoxLattice &L) {
+  const BoxWalk w = BoxWalk::make(L);
+  const RunWalk<P> rw = RunWalk<P>::make(L);
+  std::vector<int> pts(w.nL, 0);
+  for (int t = 0; t < rw.n; t++) {
+    const LatRun k = rw.run(t);
+    std::vector<int> got[P];
+    rw.first(k, [&](int r, int m) { got[r].push_back(m); });
+    rw.rest(k, [&](int r, int m) { got[r].push_back(m); });
+    for (int r = 0; r < (k.body ? P : 1); r++) {
+      const int c = k.c + r * rw.ls;
+      CHECK(c >= 0 && c < w.nL, "run walk: point %d out of range", c);
+      if (c < 0 || c >= w.nL) continue;
+      pts[c]++;
+      const BoxCopies b = w.copies(c);
+      std::vector<int> ms;
+      for (int az = 0; az < b.nz; az++)
+        for (int ay = 0; ay < b.ny; ay++)
+          for (int ax = 0; ax < b.nx; ax++)
+            ms.push_back((az ? b.oz1 : b.oz0) + (ay ? b.oy1 : b.oy0) + (ax ? b.ox1 : b.ox0));
+      CHECK(ms == got[r] && (int)ms.size() == k.nx * k.ny * (r ? 1 : k.nz),
+            "run walk: copies of point %d (dim %d p %d)", c, L.dim, P);
+    }
+  }
+  CHECK(rw.npts == w.nL, "run walk: %d points", rw.npts);
+  for (int c = 0; c < w.nL; c++) {  // a point per thread
+    const LatRun k = rw.point(c);
+    std::vector<int> got, ms;
+    rw.first(k, [&](int r, int m) { if (r == 0) got.push_back(m); });
+    rw.rest(k, [&](int r, int m) { if (r == 0) got.push_back(m); });
+    const BoxCopies b = w.copies(c);
+    for (int az = 0; az < b.nz; az++)
+      for (int ay = 0; ay < b.ny; ay++)
+        for (int ax = 0; ax < b.nx; ax++)
+          ms.push_back((az ? b.oz1 : b.oz0) + (ay ? b.oy1 : b.oy0) + (ax ? b.ox1 : b.ox0));
+    CHECK(!k.body && k.c == c && ms == got && (int)ms.size() == k.nx * k.ny * k.nz,
+          "run walk: point %d alone (dim %d p %d)", c, L.dim, P);
+  }
+  for (int c = 0; c < w.nL; c++) CHECK(pts[c] == 1, "run walk: point %d visited %d times", c, pts[c]);
+}
+
 static void check_walk(int dim, const int (&ne)[3], const int (&per)[3], int p) {
   BoxLattice L{};
   L.dim = dim;
@@ -98,6 +141,16 @@ static void check_walk(int dim, const int (&ne)[3], const int (&per)[3], int p) 
       if (w.sorted && i > 0)
         CHECK(ms[i - 1] < m, "copies of point %d not ascending (dim %d p %d)", c, dim, p);
     }
+  }
+  switch (p) {
+    case 1: check_runs<1>(L); break;
+    case 2: check_runs<2>(L); break;
+    case 3: check_runs<3>(L); break;
+    case 4: check_runs<4>(L); break;
+    case 5: check_runs<5>(L); break;
+    case 6: check_runs<6>(L); break;
+    case 7: check_runs<7>(L); break;
+    default: check_runs<8>(L); break;
   }
   for (int64_t m = 0; m < nE; m++)
     CHECK(seen[m] == 1, "node %lld visited %d times (dim %d p %d)", (long long)m, seen[m],

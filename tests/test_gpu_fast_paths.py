@@ -1,0 +1,112 @@
+"""Kernels that a rule on geometry, dimension or size selects, each against the
+general path that the same grid takes in another description:
+
+* affine 3-d right-hand side and its VJP (even-odd D and K1) against the
+  per-node geometry kernels;
+* 2-d boxes whose RK steps or CG iterations run inside one cluster against
+  the same grid without its box description (separate kernels, CSR members):
+  the steps bit for bit, the solves to the stop tolerance;
+* the line-by-line Helmholtz applies (diagonal and full metric) against dense
+  FP64 contractions in numpy.
+
+Tolerances: FP64 sums of at most 3 * 12 terms differ by rounding order, a few
+hundred eps of the largest term (1e-12); FP32 likewise (2e-5).  Solves stop at a
+relative residual of 1e-11, which leaves them within 1e-8 of each other."""
+import numpy as np
+import pytest
+
+from geoflow_b200 import _abi as A
+
+pytestmark = pytest.mark.gpu
+
+ORDERS = [1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11]
+
+
+def cuda(a, dt):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a)).to(device="cuda", dtype=dt)
+
+
+def rel(a, b):
+    import torch
+    a, b = a.double(), b.double()
+    return float((a - b).abs().max() / b.abs().max())
+
+
+def bits_equal(a, b):
+    import torch
+    i = torch.int64 if a.dtype == torch.float64 else torch.int32
+    return torch.equal(a.view(i), b.view(i))
+
+
+@pytest.mark.parametrize("ne,p,per", [([2, 3], 1, [0, 0]), ([8, 8], 3, [0, 0]), ([32, 32], 5, [0, 0]),
+                                      ([5, 7], 11, [1, 0]), ([1, 4], 6, [1, 0]), ([40, 3], 2, [0, 1]),
+                                      ([9, 6], 8, [0, 0])])
+@pytest.mark.parametrize("norm", [A.GF_NORM_INF, A.GF_NORM_EUC, A.GF_NORM_L2, A.GF_NORM_L1])
+def test_cluster_cg_equals_separate_kernels(ctx, ne, p, per, norm):
+    import torch
+    from geoflow_b200 import CGTraits, GCG, GHelmholtz, GridBox, Problem
+    g = GridBox(2, ne, p, length=[1.0, 1.7], periodic=per)
+    rng = np.random.default_rng(p)
+    first = g.members[g.class_ptr[:-1]][g.node_class]
+    b = cuda(rng.standard_normal(g.ndof()), torch.float64)
+    x0 = rng.standard_normal(g.ndof())[first]
+    lift = np.where(g.mask == 0.0, rng.standard_normal(g.ndof())[first], 0.0)
+    for pre in (A.GF_PRECOND_NONE, A.GF_PRECOND_JACOBI):
+        for xb in (None, lift):
+            res = []
+            for s in (True, False):
+                prob = Problem(ctx, g, structured=s)
+                H = GHelmholtz(prob)
+                H.set_Lap_scalar(0.3)
+                H.set_mass_scalar(2.0)
+                tr = CGTraits(maxit=4000, normtype=norm, tol=1e-11, relative=1, precond=pre)
+                cg = GCG(tr, prob)
+                x = cuda(x0, torch.float64)
+                rc = cg.solve(H, b, *([] if xb is None else [cuda(xb, torch.float64)]), x)
+                res.append((rc, cg.iter_, x, np.array(cg.get_residuals())))
+            (ra, ia, xa, ha), (rb, ib, xbb, hb) = res
+            assert ra == rb == 0
+            assert abs(ia - ib) <= max(2, ib // 20)
+            assert rel(xa, xbb) < 1e-8
+            assert abs(ha[0] - hb[0]) <= 1e-9 * hb[0]
+
+
+def test_cluster_cg_outcomes(ctx):
+    """maxit, an exact start and a non-finite right-hand side."""
+    import torch
+    from geoflow_b200 import CGTraits, GCG, GFError, GHelmholtz, GridBox, Problem
+    g = GridBox(2, [6, 6], 5)
+    prob = Problem(ctx, g)
+    H = GHelmholtz(prob)
+    H.set_mass_scalar(1.0)
+    b = cuda(np.random.default_rng(0).standard_normal(g.ndof()), torch.float64)
+    for maxit in (0, 1, 7):
+        cg = GCG(CGTraits(maxit=maxit, tol=1e-12, relative=1, precond=1), prob)
+        assert cg.solve(H, b, prob.zeros(), prob.zeros()) == 1 and cg.iter_ == maxit
+    zero = prob.zeros()
+    cg = GCG(CGTraits(maxit=50, tol=1e-12, relative=1, precond=1), prob)
+    assert cg.solve(H, zero, prob.zeros(), prob.zeros()) == 0 and cg.iter_ == 0
+    b[50] = float("nan")  # an interior node of element 1
+    with pytest.raises(GFError):
+        cg.solve(H, b, prob.zeros(), prob.zeros())
+
+
+@pytest.mark.parametrize("ne,p", [([33, 31, 33], 2), ([11, 10, 9], 7)])
+def test_multigrid_runs(ctx, ne, p):
+    """Multigrid on more than 2^18 points against the Jacobi solve of the same grid
+    without its box description."""
+    import torch
+    from geoflow_b200 import CGTraits, GCG, GHelmholtz, GridBox, Problem
+    g = GridBox(3, ne, p)
+    b = cuda(np.random.default_rng(p).standard_normal(g.ndof()), torch.float64)
+    xs = []
+    for s, pre in ((True, A.GF_PRECOND_PMG), (False, A.GF_PRECOND_JACOBI)):
+        prob = Problem(ctx, g, structured=s)
+        H = GHelmholtz(prob)
+        H.set_mass_scalar(20.0)
+        x = prob.zeros()
+        cg = GCG(CGTraits(maxit=4000, tol=1e-11, relative=1, precond=pre), prob)
+        assert cg.solve(H, b, x) == 0
+        xs.append(x)
+    assert rel(*xs) < 1e-8
