@@ -490,6 +490,16 @@ extern "C" int gf_problem_create(gf_ctx_t ctx, const gf_problem_desc *d, gf_prob
   std::memcpy(p->D, d->D, sizeof(double) * n * n);
   std::memcpy(p->W, d->W, sizeof(double) * n);
   gfk::gf_k1_matrix(n, p->D, p->W, p->K1);
+  {  // GLL bases hold this to about 100 eps of D's largest entry
+    double big = 0.0, off = 0.0;
+    for (int i = 0; i < n * n; i++) {
+      big = std::max(big, std::fabs(p->D[i]));
+      off = std::max(off, std::fabs(p->D[i] + p->D[n * n - 1 - i]));
+    }
+    p->d_antisym = off <= 1e-13 * big;
+    for (int i = 0; i < n; i++)
+      if (!(std::fabs(p->W[i] - p->W[n - 1 - i]) <= 1e-13 * std::fabs(p->W[i]))) p->d_antisym = false;
+  }
 
   // geometry
   std::vector<double> jac(N), X0(N);

@@ -44,6 +44,7 @@ struct gf_problem {
   double D[GF_MAXN * GF_MAXN];
   double W[GF_MAXN];
   double K1[GF_MAXN * GF_MAXN];  // D^T diag(W) D (affine-element apply)
+  bool d_antisym = false;  // D(n-1-l, n-1-m) = -D(l, m) and W symmetric, to rounding
   // device geometry (both precisions)
   double *egeom_d = nullptr;  // ne*(dim+1) (AFFINE)
   float *egeom_f = nullptr;

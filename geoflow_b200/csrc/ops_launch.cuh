@@ -7,6 +7,7 @@
 #include "gf_common.cuh"
 #include "k_def.cuh"
 #include "k_dudt.cuh"
+#include "k_dudt_aff.cuh"
 #include "k_helm_k1.cuh"
 #include "k_helm_tf32.cuh"
 #include "k_tensor.cuh"
@@ -163,6 +164,22 @@ struct DerivLaunch {
 template <typename T, int N, int EQN, int MODE>
 inline void launch_dudt_kernel(gf_problem *prob, T nu, const T *const *f, T *const *o,
                                const T *imass, cudaStream_t st, const RKEpi<T> &epi) {
+  if constexpr (MODE != MODE_ADVECT) {
+    // constant geometry per element and a centro-antisymmetric D (every GLL
+    // basis; a caller's own D need not be): D and K1 from one read of a line
+    if (prob->dim == 3 && prob->egeom_d && prob->d_antisym) {
+      constexpr int EPB = epb_aff<T, N>(), P = Pad<N>::P;
+      const DKBasis<T, N> B = make_dkbasis<T, N>(prob);
+      const size_t smem = sizeof(T) * aff_vols<T, EQN>() * N * N * P * EPB;
+      auto kern = k_dudt3a<T, N, EPB, EQN, MODE>;
+      set_smem(kern, smem);
+      prob->launches++;
+      kern<<<(unsigned)((prob->ne + EPB - 1) / EPB), dim3(N * N, EPB), smem, st>>>(
+          B, geom_of<T>(prob).egeom, prob->ne, nu, f[0], f[1], f[2], f[3], imass, o[0], o[1], o[2],
+          epi);
+      return;
+    }
+  }
   const Basis<T, N> B = make_basis<T, N>(prob);
   const Geom<T> g = geom_of<T>(prob);
   constexpr int P = Pad<N>::P;

@@ -39,6 +39,58 @@ def bits_equal(a, b):
     return torch.equal(a.view(i), b.view(i))
 
 
+@pytest.mark.parametrize("p", ORDERS)
+@pytest.mark.parametrize("eqn", [A.GF_EQN_ADVECT, A.GF_EQN_BURGERS, A.GF_EQN_HEAT])
+def test_affine_rhs_equals_nodal(ctx, p, eqn):
+    import torch
+    from geoflow_b200 import GBurgers, GridBox, Problem
+    g = GridBox(3, [3, 2, 2], p, length=[1.0, 0.7, 1.9], periodic=[1, 0, 1])
+    pa, pn = Problem(ctx, g, dirichlet_mask=False), Problem(ctx, g, dirichlet_mask=False,
+                                                            geometry="regular")
+    rng = np.random.default_rng(p)
+    ns = 3 if eqn == A.GF_EQN_BURGERS else 1
+    u0 = [rng.standard_normal(g.ndof()) for _ in range(ns)]
+    c0 = [rng.standard_normal(g.ndof()) for _ in range(3)] if eqn == A.GF_EQN_ADVECT else None
+    for dt, tol in ((torch.float64, 1e-12), (torch.float32, 2e-5)):
+        u = [cuda(a, dt) for a in u0]
+        c = [cuda(a, dt) for a in c0] if c0 else None
+        out = []
+        for prob in (pa, pn):
+            o = prob.zeros(dt, ncomp=ns)
+            GBurgers(prob, eqn, 0.03).dudt(u, c, o)
+            out.append(o)
+        for a, b in zip(*out):
+            assert rel(a, b) < tol, (dt, rel(a, b))
+    # the VJP (FP64)
+    u, lam = [cuda(a, torch.float64) for a in u0], [cuda(rng.standard_normal(g.ndof()), torch.float64)
+                                                   for _ in range(ns)]
+    c = [cuda(a, torch.float64) for a in c0] if c0 else None
+    out = []
+    for prob in (pa, pn):
+        o = prob.zeros(ncomp=ns)
+        GBurgers(prob, eqn, 0.03).dudt_vjp(u, c, lam, o)
+        out.append(o)
+    for a, b in zip(*out):
+        assert rel(a, b) < 1e-12, rel(a, b)
+
+
+def test_rhs_with_an_asymmetric_derivative_matrix(ctx):
+    """A caller's D that is not centro-antisymmetric keeps the general kernels."""
+    import torch
+    from geoflow_b200 import GBurgers, GridBox, Problem
+    g = GridBox(3, [2, 2, 2], 4)
+    g.D = g.D * (1.0 + 0.1 * np.random.default_rng(0).standard_normal(g.D.size))
+    u = [cuda(np.random.default_rng(k).standard_normal(g.ndof()), torch.float64) for k in range(3)]
+    out = []
+    for geom in ("affine", "regular"):
+        prob = Problem(ctx, g, geometry=geom)
+        o = prob.zeros(ncomp=3)
+        GBurgers(prob, A.GF_EQN_BURGERS, 0.1).dudt(u, None, o)
+        out.append(o)
+    for a, b in zip(*out):
+        assert rel(a, b) < 1e-12
+
+
 @pytest.mark.parametrize("ne,p,per", [([2, 3], 1, [0, 0]), ([8, 8], 3, [0, 0]), ([32, 32], 5, [0, 0]),
                                       ([5, 7], 11, [1, 0]), ([1, 4], 6, [1, 0]), ([40, 3], 2, [0, 1]),
                                       ([9, 6], 8, [0, 0])])
