@@ -326,11 +326,9 @@ __device__ void en_rhs_elem(const LaneTeam &tm, const EnArgs &a, int mi, const E
   const int nv = a.eqn == GF_EQN_ADVECT ? M.nxy : 0;
   const T *c0 = (const T *)M.c[0], *c1 = (const T *)M.c[1], *c2 = (const T *)M.c[2];
   if (fin)
-    def_element<T, N, 2, LoadFinal<T>, T>(tm, B, g, e, DEF_DUDT, nu, nullptr, T(0), nullptr, 0,
-                                          ldf, nv, c0, c1, c2, 0, imass, out, slice);
+    def_element<T, N, 2, LoadFinal<T>, T>(tm, B, g, e, DEF_DUDT, nu, ldf, nv, c0, c1, c2, 0, imass, out, slice);
   else
-    def_element<T, N, 2, LoadStage<T>, T>(tm, B, g, e, DEF_DUDT, nu, nullptr, T(0), nullptr, 0,
-                                          lds, nv, c0, c1, c2, 0, imass, out, slice);
+    def_element<T, N, 2, LoadStage<T>, T>(tm, B, g, e, DEF_DUDT, nu, lds, nv, c0, c1, c2, 0, imass, out, slice);
 }
 
 // Element phase of an RK stage: K_stage = dudt(stage input), or for the

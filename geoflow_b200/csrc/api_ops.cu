@@ -171,15 +171,11 @@ extern "C" int gf_deriv(gf_problem_t prob, int dtype, const void *u, int idir, v
   if (prob->geom >= GF_GEOM_DEFORMED) {  // sum_j dXi_j/dX_idir D_j u
     rc = dtype == GF_F64
              ? dispatch_n<DefLaunch<double, LoadE<double>>::template F>(
-                   prob->n, prob, (int)DEF_DERIV, 0.0, (const double *)nullptr, 0.0,
-                   (const double *)nullptr, 0, LoadE<double>{(const double *)u}, 0,
-                   (const double *const *)nullptr, idir, (double *)du, ctx->stream,
-                   (const double *)nullptr)
+                   prob->n, prob, (int)DEF_DERIV, 0.0, LoadE<double>{(const double *)u}, 0,
+                   (const double *const *)nullptr, idir, (double *)du, ctx->stream)
              : dispatch_n<DefLaunch<float, LoadE<float>>::template F>(
-                   prob->n, prob, (int)DEF_DERIV, 0.0f, (const float *)nullptr, 0.0f,
-                   (const float *)nullptr, 0, LoadE<float>{(const float *)u}, 0,
-                   (const float *const *)nullptr, idir, (float *)du, ctx->stream,
-                   (const double *)nullptr);
+                   prob->n, prob, (int)DEF_DERIV, 0.0f, LoadE<float>{(const float *)u}, 0,
+                   (const float *const *)nullptr, idir, (float *)du, ctx->stream);
   } else {
     rc = dtype == GF_F64
              ? deriv_common<double>(prob, (const double *)u, idir, 0, 1, 0, (double *)du)
@@ -210,49 +206,6 @@ extern "C" int gf_grefdiv(gf_problem_t prob, int dtype, const void *const *u, in
 // ---------------------------------------------------------------------
 // advection and Burgers RHS
 // ---------------------------------------------------------------------
-// Deformed / embedded elements: one k_def launch per evolved component,
-// the reference gradient shared by advection and diffusion.  f as for
-// launch_dudt: ADVECT {p, c0, c1, c2}, BURGERS {u0, u1, u2}, HEAT {u}.
-template <typename T>
-static int launch_def_dudt(gf_problem *prob, int eqn, int mode, T nu, const T *const *f,
-                           T *const *o, cudaStream_t st) {
-  const int nv = prob->nxy;
-  if (eqn == GF_EQN_ADVECT) {
-    const T *c[3] = {f[1], f[2], f[3]};
-    return dispatch_n<DefLaunch<T, LoadE<T>>::template F>(
-        prob->n, prob, mode == MODE_ADVECT ? (int)DEF_ADVECT : (int)DEF_DUDT, nu, (const T *)nullptr,
-        T(0), (const T *)nullptr, 0, LoadE<T>{f[0]}, nv, (const T *const *)c, 0, o[0], st,
-        (const double *)nullptr);
-  }
-  if (eqn == GF_EQN_HEAT)
-    return dispatch_n<DefLaunch<T, LoadE<T>>::template F>(
-        prob->n, prob, (int)DEF_DUDT, nu, (const T *)nullptr, T(0), (const T *)nullptr, 0,
-        LoadE<T>{f[0]}, 0, (const T *const *)nullptr, 0, o[0], st, (const double *)nullptr);
-  for (int k = 0; k < nv; k++) {  // Burgers: the velocity is the state
-    int rc = dispatch_n<DefLaunch<T, LoadE<T>>::template F>(
-        prob->n, prob, (int)DEF_DUDT, nu, (const T *)nullptr, T(0), (const T *)nullptr, 0,
-        LoadE<T>{f[k]}, nv, f, 0, o[k], st, (const double *)nullptr);
-    if (rc) return rc;
-  }
-  return GF_OK;
-}
-
-template <typename T>
-int launch_dudt(gf_problem *prob, int eqn, int mode, T nu, const T *const *f, T *const *o,
-                cudaStream_t st, const gfk::RKEpi<T> *epi) {
-  if (prob->geom >= GF_GEOM_DEFORMED) {
-    if (mode == MODE_EULER) return GF_ERR_UNSUPPORTED;
-    return launch_def_dudt<T>(prob, eqn, mode, nu, f, o, st);
-  }
-  const RKEpi<T> none{};
-  return dispatch_n<DudtLaunch<T>::template F>(prob->n, prob, eqn, mode, nu, f, o, st,
-                                               epi ? *epi : none);
-}
-template int launch_dudt<double>(gf_problem *, int, int, double, const double *const *,
-                                 double *const *, cudaStream_t, const gfk::RKEpi<double> *);
-template int launch_dudt<float>(gf_problem *, int, int, float, const float *const *,
-                                float *const *, cudaStream_t, const gfk::RKEpi<float> *);
-
 extern "C" int gf_advect_apply(gf_problem_t prob, int dtype, const void *p, int ncomp,
                                const void *const *c, void *po) {
   if (!prob) return GF_ERR_ARG;

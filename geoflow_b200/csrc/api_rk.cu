@@ -92,8 +92,10 @@ struct AdvLaunch {
                    cudaStream_t st) {
       const Basis<T, N> B = make_basis<T, N>(prob);
       prob->launches++;
-      k_adv_def<T, N, LoadE<T>><<<(unsigned)((prob->ne + 3) / 4), 128, 0, st>>>(
-          B, prob->ne, LoadE<T>{u}, b0, b1, out);
+      constexpr int EPB = epb2l<N>();
+      k_adv_def<T, N, EPB, LoadE<T>>
+          <<<(unsigned)((prob->ne + EPB - 1) / EPB), 2 * N * EPB, 0, st>>>(B, prob->ne, LoadE<T>{u},
+                                                                          b0, b1, out);
       return GF_OK;
     }
   };

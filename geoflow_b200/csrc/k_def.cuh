@@ -45,9 +45,9 @@ template <> inline DefGeom<float> def_of<float>(const gf_problem *p) {
                         p->nlocal};
 }
 
-enum { DEF_HELM = 0, DEF_DUDT = 1, DEF_ADVECT = 2, DEF_DERIV = 3 };
+enum { DEF_DUDT = 1, DEF_ADVECT = 2, DEF_DERIV = 3 };
 
-// mode DEF_HELM: uo = p L u (+ q M u); DEF_DUDT: uo = Minv(-nu L u - adv)
+// def_element: mode DEF_DUDT: uo = Minv(-nu L u - adv)
 // (heat when nv == 0); DEF_ADVECT: uo = adv = M sum_k c_k du/dx_k;
 // DEF_DERIV: uo = du/dx_{idir}.  nv velocity components c0..c2.
 // The threads that share one element: the whole block (k_def), or a group
@@ -79,10 +79,7 @@ struct OutPtr {
 // is the same whichever thread of whichever team computes it.
 template <typename T, int N, int DIM, class LD, typename TO, class BB, class TM, class OUT>
 __device__ __forceinline__ void def_element(const TM &tm, const BB &B, const DefGeom<T> &g,
-                                            int64_t e, int mode,
-                                            T p, const T *__restrict__ pvec, T q,
-                                            const T *__restrict__ qvec, int use_mass, const LD &ld,
-                                            int nv, const T *__restrict__ c0,
+                                            int64_t e, int mode, T nu, const LD &ld, int nv, const T *__restrict__ c0,
                                             const T *__restrict__ c1, const T *__restrict__ c2,
                                             int idir, const T *__restrict__ imass,
                                             const OUT &uo, T *smem) {
@@ -135,7 +132,6 @@ __device__ __forceinline__ void def_element(const TM &tm, const BB &B, const Def
         T gj = T(0);
 #pragma unroll
         for (int i = 0; i < DIM; i++) gj += sd[i * NE + a] * g.G[gpack(i, j, DIM) * nl + node];
-        if (mode == DEF_HELM && pvec) gj *= pvec[node];
         sg[j * NE + a] = gj;
       }
     }
@@ -174,21 +170,9 @@ __device__ __forceinline__ void def_element(const TM &tm, const BB &B, const Def
       for (int m = 1; m < N; m++) s = fma(B.D[m + li[j] * N], sg[j * NE + b0 + m * st[j]], s);
       o = j == 0 ? s : o + s;
     }
-    if (mode == DEF_HELM) {
-      if (!pvec) o *= p;
-      if (use_mass) {
-        T mass = B.W[li[0]] * B.W[li[1]];
-        if (DIM == 3) mass *= B.W[li[2]];
-        T t = (mass * g.J[node]) * su[a];
-        t *= qvec ? qvec[node] : q;
-        o += t;
-      }
-      uo(node, (TO)o);
-    } else {  // DEF_DUDT
-      o *= p;  // p = nu
-      const T r = nv > 0 ? T(-1) * o + T(-1) * su[a] : T(-1) * o;
-      uo(node, (TO)(imass[node] * r));
-    }
+    o *= nu;
+    const T r = nv > 0 ? T(-1) * o + T(-1) * su[a] : T(-1) * o;
+    uo(node, (TO)(imass[node] * r));
   }
 }
 
@@ -250,19 +234,164 @@ __device__ __forceinline__ void adv_element(const TM &tm, const BB &B, int64_t e
   }
 }
 
+// ---- Helmholtz apply, line by line ----
+// def_prod / embed_prod with each thread owning an x-, a y- and a z-line of the
+// element (k_tensor.cuh): D_x u and D_y u go through shared memory to the owner
+// of the node's z-column, which reads the metric planes once and coalesced,
+// forms sum_i G_ij D_i u and returns the x- and y-parts for the transposed
+// contractions.  15 shared-memory words per node; def_element, one thread per
+// node, takes 6 N (and D at a run-time row: a replay per distinct row in the
+// parameter bank): 100 us at 16x15x14 elements, p = 7, FP64, against a floor of
+// 19 us for the planes.
+template <typename T, int N, int EPB, class LD>
+__global__ void __launch_bounds__(N *N *EPB)
+    k_helm3d_full(const __grid_constant__ Basis<T, N> B, const DefGeom<T> g, int64_t ne, T p,
+                  const T *__restrict__ pvec, T q, const T *__restrict__ qvec, int use_mass,
+                  const LD ld, T *__restrict__ uo, const double *__restrict__ stop) {
+  if (stop && stop[0] != 0.0) return;
+  constexpr int P = Pad<N>::P, PLANE = N * P, VOL = N * PLANE, NN = N * N, NNN = N * N * N;
+  extern __shared__ __align__(16) unsigned char smem_def[];
+  T *su = reinterpret_cast<T *>(smem_def) + threadIdx.y * 3 * VOL;
+  T *sx = su + VOL, *sy = su + 2 * VOL;
+  const int t = threadIdx.x, a0 = t % N, a1 = t / N;
+  const int64_t e = (int64_t)blockIdx.x * EPB + threadIdx.y;
+  const bool active = e < ne;
+  const int64_t base = e * NNN, nl = g.nlocal;
+  const int xl = a1 * PLANE + a0 * P, yl = a1 * PLANE + a0, zl = a1 * P + a0;
+  T ru[N];
+  if (active) {
+    typename LD::value_type lv[N];
+    ld.template zline<N>(e, a0, a1, lv);
+#pragma unroll
+    for (int k = 0; k < N; k++) ru[k] = (T)lv[k];
+  } else {
+#pragma unroll
+    for (int k = 0; k < N; k++) ru[k] = T(0);
+  }
+#pragma unroll
+  for (int k = 0; k < N; k++) su[zl + k * PLANE] = ru[k];
+  __syncthreads();
+  T a[3][N], gz[N];
+#pragma unroll
+  for (int m = 0; m < N; m++) {
+    a[0][m] = su[xl + m];
+    a[1][m] = su[yl + m * P];
+    a[2][m] = ru[m];
+  }
+  lines_D<T, N, 3, false>(B.D, a, [&](int l, int i, T v) {
+    if (l == 0) sx[xl + i] = v;
+    else if (l == 1) sy[yl + i * P] = v;
+    else gz[i] = v;
+  });
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    T gx = T(0), gy = T(0), g2 = T(0);
+    if (active) {
+      const int64_t node = base + k * NN + t;
+      const T dx = sx[zl + k * PLANE], dy = sy[zl + k * PLANE], dz = gz[k];
+      const T pv = pvec ? pvec[node] : p;
+      const T g01 = g.G[nl + node], g02 = g.G[2 * nl + node], g12 = g.G[4 * nl + node];
+      gx = pv * (dx * g.G[node] + dy * g01 + dz * g02);
+      gy = pv * (dx * g01 + dy * g.G[3 * nl + node] + dz * g12);
+      g2 = pv * (dx * g02 + dy * g12 + dz * g.G[5 * nl + node]);
+    }
+    sx[zl + k * PLANE] = gx;
+    sy[zl + k * PLANE] = gy;
+    gz[k] = g2;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < N; m++) {
+    a[0][m] = sx[xl + m];
+    a[1][m] = sy[yl + m * P];
+    a[2][m] = gz[m];
+  }
+  lines_D<T, N, 3, true>(B.D, a, [&](int l, int i, T v) {
+    if (l == 0) sx[xl + i] = v;
+    else if (l == 1) sy[yl + i * P] = v;
+    else gz[i] = v;
+  });
+  __syncthreads();
+  if (active) {
+    const T w2 = B.W[a0] * B.W[a1];
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+      const int64_t node = base + k * NN + t;
+      T o = (sx[zl + k * PLANE] + sy[zl + k * PLANE]) + gz[k];
+      if (use_mass)
+        o = fma(B.W[k] * w2 * g.J[node] * (qvec ? qvec[node] : q), su[zl + k * PLANE], o);
+      uo[node] = o;
+    }
+  }
+}
+
+// 2-d (deformed or embedded), 2 N threads per element as in k_helm2d.
+template <typename T, int N, int EPB, class LD>
+__global__ void __launch_bounds__(2 * N *EPB)
+    k_helm2d_full(const __grid_constant__ Basis<T, N> B, const DefGeom<T> g, int64_t ne, T p,
+                  const T *__restrict__ pvec, T q, const T *__restrict__ qvec, int use_mass,
+                  const LD ld, T *__restrict__ uo, const double *__restrict__ stop) {
+  if (stop && stop[0] != 0.0) return;
+  constexpr int P = Pad<N>::P, AREA = N * P, NN = N * N, NT = 2 * N * EPB;
+  __shared__ T su[EPB * AREA], sx[EPB * AREA], sy[EPB * AREA], sW[N];
+  const int64_t e0 = (int64_t)blockIdx.x * EPB, n0 = e0 * NN, nl = g.nlocal;
+  const int nel = ne - e0 < EPB ? (int)(ne - e0) : EPB;
+  const int t = threadIdx.x, el = t / (2 * N), l = t - el * 2 * N;
+  const bool xdir = l < N, on = el < nel;
+  const int s0 = el * AREA + (xdir ? l * P : l - N), st = xdir ? 1 : P;
+  T *w = xdir ? sx : sy;
+  T a[N], d[N];
+  if (t < N) sW[t] = B.W[t];
+  for (int i = t; i < nel * NN; i += NT) {
+    const int ie = i / NN, b = i - ie * NN, y = b / N, x = b - y * N;
+    su[ie * AREA + y * P + x] = (T)ld.template point2<N>(e0 + ie, x, y);
+  }
+  __syncthreads();
+  if (on) {
+#pragma unroll
+    for (int m = 0; m < N; m++) a[m] = su[s0 + m * st];
+    line_D<T, N>(B.D, a, d);
+#pragma unroll
+    for (int m = 0; m < N; m++) w[s0 + m * st] = d[m];
+  }
+  __syncthreads();
+  for (int i = t; i < nel * NN; i += NT) {
+    const int ie = i / NN, b = i - ie * NN, y = b / N, x = b - y * N;
+    const int s = ie * AREA + y * P + x;
+    const int64_t node = n0 + i;
+    const T dx = sx[s], dy = sy[s], pv = pvec ? pvec[node] : p, g01 = g.G[nl + node];
+    sx[s] = pv * (dx * g.G[node] + dy * g01);
+    sy[s] = pv * (dx * g01 + dy * g.G[2 * nl + node]);
+  }
+  __syncthreads();
+  if (on) {
+#pragma unroll
+    for (int m = 0; m < N; m++) a[m] = w[s0 + m * st];
+    line_DT<T, N>(B.D, a, d);
+#pragma unroll
+    for (int m = 0; m < N; m++) w[s0 + m * st] = d[m];
+  }
+  __syncthreads();
+  for (int i = t; i < nel * NN; i += NT) {
+    const int ie = i / NN, b = i - ie * NN, y = b / N, x = b - y * N;
+    const int s = ie * AREA + y * P + x;
+    const int64_t node = n0 + i;
+    T o = sx[s] + sy[s];
+    if (use_mass) o = fma(sW[y] * sW[x] * g.J[node] * (qvec ? qvec[node] : q), su[s], o);
+    uo[node] = o;
+  }
+}
+
 template <typename T, int N, int DIM, class LD, typename TO>
 __global__ void __launch_bounds__(256)
-    k_def(const __grid_constant__ Basis<T, N> B, const DefGeom<T> g, int64_t ne, int mode, T p,
-          const T *__restrict__ pvec, T q, const T *__restrict__ qvec, int use_mass, const LD ld,
-          int nv, const T *__restrict__ c0, const T *__restrict__ c1, const T *__restrict__ c2,
-          int idir, const T *__restrict__ imass, TO *__restrict__ uo,
-          const double *__restrict__ stop) {
-  if (stop && stop[0] != 0.0) return;
+    k_def(const __grid_constant__ Basis<T, N> B, const DefGeom<T> g, int64_t ne, int mode, T nu,
+          const LD ld, int nv, const T *__restrict__ c0, const T *__restrict__ c1, const T *__restrict__ c2,
+          int idir, const T *__restrict__ imass, TO *__restrict__ uo) {
   extern __shared__ __align__(16) unsigned char smem_def[];
   const int64_t e = blockIdx.x;
   if (e >= ne) return;
-  def_element<T, N, DIM, LD, TO>(BlockTeam{}, B, g, e, mode, p, pvec, q, qvec, use_mass, ld, nv, c0,
-                                 c1, c2, idir, imass, OutPtr<TO>{uo},
+  def_element<T, N, DIM, LD, TO>(BlockTeam{}, B, g, e, mode, nu, ld, nv, c0, c1, c2, idir, imass, OutPtr<TO>{uo},
                                  reinterpret_cast<T *>(smem_def));
 }
 
@@ -280,17 +409,41 @@ __global__ void k_adv_coef(const __grid_constant__ Basis<T, N> B, const DefGeom<
   }
 }
 
-// adv_element on one 2-d problem: one element per warp, four per block.
-template <typename T, int N, class LD>
-__global__ void __launch_bounds__(128)
+// adv_element on one 2-d problem, bit for bit: 2 N threads per element, one
+// x-line or y-line each (k_helm2d), with the chains of adv_element; then node by
+// node.
+template <typename T, int N, int EPB, class LD>
+__global__ void __launch_bounds__(2 * N *EPB)
     k_adv_def(const __grid_constant__ Basis<T, N> B, int64_t ne, const LD ld,
               const T *__restrict__ b0, const T *__restrict__ b1, T *__restrict__ out) {
-  __shared__ T su[4][N * N];
-  const int w = threadIdx.x >> 5;
-  const int64_t e = (int64_t)blockIdx.x * 4 + w;
-  if (e >= ne) return;  // whole warps
-  adv_element<T, N>(LaneTeam{(int)(threadIdx.x & 31), 32, 0xffffffffu}, B, e, ld, b0, b1,
-                    OutPtr<T>{out}, su[w]);
+  constexpr int P = Pad<N>::P, AREA = N * P, NN = N * N, NT = 2 * N * EPB;
+  __shared__ T su[EPB * AREA], sx[EPB * AREA], sy[EPB * AREA];
+  const int64_t e0 = (int64_t)blockIdx.x * EPB, n0 = e0 * NN;
+  const int nel = ne - e0 < EPB ? (int)(ne - e0) : EPB;
+  const int t = threadIdx.x, el = t / (2 * N), l = t - el * 2 * N;
+  for (int i = t; i < nel * NN; i += NT) {
+    const int ie = i / NN, b = i - ie * NN, y = b / N, x = b - y * N;
+    su[ie * AREA + y * P + x] = (T)ld.template point2<N>(e0 + ie, x, y);
+  }
+  __syncthreads();
+  if (el < nel) {
+    const bool xdir = l < N;
+    const int s0 = el * AREA + (xdir ? l * P : l - N), st = xdir ? 1 : P;
+    T *w = xdir ? sx : sy;
+    T a[N], d[N];
+#pragma unroll
+    for (int m = 0; m < N; m++) a[m] = su[s0 + m * st];
+    line_D<T, N>(B.D, a, d);
+#pragma unroll
+    for (int m = 0; m < N; m++) w[s0 + m * st] = d[m];
+  }
+  __syncthreads();
+  for (int i = t; i < nel * NN; i += NT) {
+    const int ie = i / NN, b = i - ie * NN, y = b / N, x = b - y * N;
+    const int s = ie * AREA + y * P + x;
+    const T c0 = b0[n0 + i], c1 = b1[n0 + i];
+    out[n0 + i] = fma(c1, sy[s], c0 * sx[s]);
+  }
 }
 
 }  // namespace gfk

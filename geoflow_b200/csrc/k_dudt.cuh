@@ -19,7 +19,7 @@ enum { MODE_DUDT = 0, MODE_ADVECT = 1, MODE_EULER = 2 };
 
 // MODE_EULER: the right-hand side K = dudt of each evolved component is
 // not stored; the kernel stores the SSP substep's update before its Smooth
-// instead, with the stage arithmetic of k_dss_rk_box_n (FUSE_EULER):
+// instead, with the stage arithmetic of the class pass (k_dss.cuh RK_EULER):
 //   x = dt K + 1 uin;  x = a x + b y (if y);  x = a2 x + b2 y2 (if y2)
 // (gexrk_stepper.ipp:533-780, 809-819), K rounded to T first, so the
 // following Smooth gives the same bits as the fused update-and-Smooth pass.
@@ -227,77 +227,102 @@ __global__ void __launch_bounds__(N *N *EPB, (sizeof(T) == 4 && MODE != MODE_EUL
   }
 }
 
-// 2-d variant, one thread per node.
-template <typename T, int N, int EPB, int EQN, int MODE>
-__global__ void __launch_bounds__(N *N *EPB)
-    k_dudt2d(const __grid_constant__ Basis<T, N> B, const Geom<T> g, int64_t ne, T nu,
-             const T *__restrict__ f0, const T *__restrict__ f1, const T *__restrict__ f2,
-             const T *__restrict__ f3, const T *__restrict__ imass, T *__restrict__ o0,
-             T *__restrict__ o1, T *__restrict__ o2, const RKEpi<T> epi) {
-  (void)epi;  // the 2-d kernel has no fused update (MODE_EULER is 3-d only)
+// 2-d variant: 2 N threads per element, one x-line or y-line each (k_helm2d in
+// k_tensor.cuh, with the reason); with a diagonal metric both the advection and
+// the diffusion term of a direction stay on its line, so a component costs two
+// reads of a line, one write and two barriers.
+
+// shared-memory words of one element: the fields, and the x- and y-terms of
+// each evolved component
+template <int N, int EQN> constexpr int dudt2_words() {
+  return ((EQN == GF_EQN_ADVECT ? 3 : (EQN == GF_EQN_BURGERS ? 2 : 1)) +
+          (EQN == GF_EQN_BURGERS ? 4 : 2)) * N * Pad<N>::P;
+}
+
+// Elements e0 .. e0 + nel - 1 by one block of at least 2 N nel threads; sm holds
+// nel dudt2_words, sW the weights (loaded by the caller).  The fields are not
+// __restrict__: a kernel that has written them in an earlier phase calls this.
+template <typename T, int N, int EQN, int MODE>
+__device__ __forceinline__ void dudt2d_group(const Basis<T, N> &B, const Geom<T> &g, int64_t e0,
+                                             int nel, T nu, const T *f0, const T *f1, const T *f2,
+                                             const T *imass, T *o0, T *o1, T *sm, const T *sW) {
   constexpr int NF = EQN == GF_EQN_ADVECT ? 3 : (EQN == GF_EQN_BURGERS ? 2 : 1);
   constexpr int NC = EQN == GF_EQN_BURGERS ? 2 : 1;
   constexpr int P = Pad<N>::P, AREA = N * P, NN = N * N;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *s = reinterpret_cast<T *>(smem_raw) + threadIdx.y * (NF + 2) * AREA;
-  T *sgx = s + NF * AREA, *sgy = s + (NF + 1) * AREA;
-  const int t = threadIdx.x;
-  const int64_t e = (int64_t)blockIdx.x * EPB + threadIdx.y;
-  const bool active = e < ne;
-  const int i = t % N, j = t / N;
-  const int64_t node = e * NN + t;
+  const int FS = nel * AREA;  // one field of the group
+  T *su = sm, *sx = su + NF * FS, *sy = sx + NC * FS;
+  const int64_t n0 = e0 * NN;
+  const int t = threadIdx.x, el = t / (2 * N), l = t - el * 2 * N;
   const T *fin[3] = {f0, f1, f2};
-  T *fout[2] = {o0, o1};
-  (void)f3;
-  NodeGeom<T, 2> ng;
-  ng.X[0] = ng.X[1] = ng.J = T(0);
-  if (active) {
-    elem_geom<T, 2>(g, e, ng);
-    node_geom<T, 2>(g, node, ng);
-  }
+  for (int i = t; i < nel * NN; i += blockDim.x) {
+    const int ie = i / NN, b = i - ie * NN, y = b / N, x = b - y * N;
 #pragma unroll
-  for (int f = 0; f < NF; f++) s[f * AREA + j * P + i] = active ? fin[f][node] : T(0);
-  const T mass = B.W[j] * B.W[i] * ng.J;
+    for (int f = 0; f < NF; f++) su[f * FS + ie * AREA + y * P + x] = fin[f][n0 + i];
+  }
   __syncthreads();
-#pragma unroll 1
-  for (int c = 0; c < NC; c++) {
-    const T *su = s + c * AREA;
-    T dx = B.D[i] * su[j * P];
-    T dy = B.D[j] * su[i];
+  if (el < nel) {
+    const bool xdir = l < N;
+    const int ln = xdir ? l : l - N;
+    const int s0 = el * AREA + (xdir ? ln * P : ln), st = xdir ? 1 : P;
+    const int64_t g0 = n0 + el * NN + (xdir ? ln * N : ln);
+    T *w = xdir ? sx : sy;
+    // mass X and the velocity along the line
+    T mx[N], X[N], v[N];
+    NodeGeom<T, 2> ng;
+    elem_geom<T, 2>(g, e0 + el, ng);
+    const int fv = EQN == GF_EQN_ADVECT ? (xdir ? 1 : 2) : (xdir ? 0 : 1);
 #pragma unroll
-    for (int m = 1; m < N; m++) {
-      dx = fma(B.D[i + m * N], su[j * P + m], dx);
-      dy = fma(B.D[j + m * N], su[m * P + i], dy);
+    for (int m = 0; m < N; m++) {
+      node_geom<T, 2>(g, g0 + m * (xdir ? 1 : N), ng);
+      X[m] = xdir ? ng.X[0] : ng.X[1];
+      mx[m] = sW[ln] * B.W[m] * ng.J * X[m];
+      v[m] = EQN == GF_EQN_HEAT ? T(0) : su[fv * FS + s0 + m * st];
     }
-    T adv = T(0);
-    if (EQN != GF_EQN_HEAT) {
-      const int cb = EQN == GF_EQN_ADVECT ? 1 : 0;
-      T po = (dx * ng.X[0]) * s[(cb + 0) * AREA + j * P + i];
-      po += (dy * ng.X[1]) * s[(cb + 1) * AREA + j * P + i];
-      adv = po * mass;
-    }
-    if (MODE == MODE_ADVECT) {
-      if (active) fout[c][node] = adv;
-      continue;
-    }
-    sgx[j * P + i] = mass * (dx * (ng.X[0] * ng.X[0]));
-    sgy[j * P + i] = mass * (dy * (ng.X[1] * ng.X[1]));
-    __syncthreads();
-    T ox = B.D[i * N] * sgx[j * P];
-    T oy = B.D[j * N] * sgy[i];
 #pragma unroll
-    for (int m = 1; m < N; m++) {
-      ox = fma(B.D[m + i * N], sgx[j * P + m], ox);
-      oy = fma(B.D[m + j * N], sgy[m * P + i], oy);
-    }
-    __syncthreads();
-    if (active) {
-      T L = ox + oy;
-      if (nu != T(1)) L *= nu;
-      T rhs = T(-1) * L + T(-1) * adv;
-      fout[c][node] = imass[node] * rhs;
+    for (int c = 0; c < NC; c++) {
+      T a[N], d[N];
+#pragma unroll
+      for (int m = 0; m < N; m++) a[m] = su[c * FS + s0 + m * st];
+      line_D<T, N>(B.D, a, d);
+      T r[N];
+      if constexpr (MODE == MODE_ADVECT) {
+#pragma unroll
+        for (int m = 0; m < N; m++) r[m] = mx[m] * d[m] * v[m];
+      } else {
+#pragma unroll
+        for (int m = 0; m < N; m++) a[m] = mx[m] * X[m] * d[m];
+        line_DT<T, N>(B.D, a, r);
+#pragma unroll
+        for (int m = 0; m < N; m++)
+          r[m] = EQN == GF_EQN_HEAT ? nu * r[m] : fma(mx[m] * d[m], v[m], nu * r[m]);
+      }
+#pragma unroll
+      for (int m = 0; m < N; m++) w[c * FS + s0 + m * st] = r[m];
     }
   }
+  __syncthreads();
+  for (int i = t; i < nel * NN; i += blockDim.x) {
+    const int ie = i / NN, b = i - ie * NN, y = b / N, x = b - y * N;
+    const int s = ie * AREA + y * P + x;
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+      const T r = sx[c * FS + s] + sy[c * FS + s];
+      (c == 0 ? o0 : o1)[n0 + i] = MODE == MODE_ADVECT ? r : -imass[n0 + i] * r;
+    }
+  }
+}
+
+template <typename T, int N, int EPB, int EQN, int MODE>
+__global__ void __launch_bounds__(2 * N *EPB)
+    k_dudt2d(const __grid_constant__ Basis<T, N> B, const Geom<T> g, int64_t ne, T nu,
+             const T *__restrict__ f0, const T *__restrict__ f1, const T *__restrict__ f2,
+             const T *__restrict__ imass, T *__restrict__ o0, T *__restrict__ o1) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ T sW[N];
+  if (threadIdx.x < N) sW[threadIdx.x] = B.W[threadIdx.x];
+  const int64_t e0 = (int64_t)blockIdx.x * EPB;
+  dudt2d_group<T, N, EQN, MODE>(B, g, e0, ne - e0 < EPB ? (int)(ne - e0) : EPB, nu, f0, f1, f2,
+                                imass, o0, o1, reinterpret_cast<T *>(smem_raw), sW);
 }
 
 }  // namespace gfk

@@ -9,9 +9,8 @@
 // n.  Rows are padded to an odd length so that x-line reads by consecutive
 // threads fall in distinct banks.
 //
-// These kernels implement the arithmetic of GHelmholtz::reg_prod
-// (sem/ghelmholtz.ipp:309-378): gdu_k = Mass (G_kk (D_k u)), uo =
-// sum_k D_k^T gdu_k, times a scalar p, plus q M u.
+// These kernels implement GHelmholtz::reg_prod (sem/ghelmholtz.ipp:309-378):
+// gdu_k = Mass (G_kk (D_k u)), uo = sum_k D_k^T gdu_k, times p, plus q M u.
 #pragma once
 #include "gf_common.cuh"
 #include "k_maps.cuh"
@@ -44,8 +43,29 @@ __device__ __forceinline__ void line_DT(const T *__restrict__ D, const T (&a)[N]
   }
 }
 
+// L lines at once, one read of a matrix entry for all of them: out(l, i,
+// sum_m A(i, m) a[l][m]), A = D, or D^T with TR; same sums in the same order as
+// line_D and line_DT.  In FP64 an entry is a load from the parameter bank, 6 N^2
+// of them per thread with a line at a time: the full-metric apply at N = 8 took
+// 70 us that way and 43 with three lines.
+template <typename T, int N, int L, bool TR, class OUT>
+__device__ __forceinline__ void lines_D(const T *__restrict__ D, const T (&a)[L][N], OUT out) {
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    T s[L];
+#pragma unroll
+    for (int m = 0; m < N; m++) {
+      const T c = TR ? D[m + i * N] : D[i + m * N];
+#pragma unroll
+      for (int l = 0; l < L; l++) s[l] = m == 0 ? c * a[l][0] : fma(c, a[l][m], s[l]);
+    }
+#pragma unroll
+    for (int l = 0; l < L; l++) out(l, i, s[l]);
+  }
+}
+
 template <int N> constexpr int epb3() {
-  return N <= 2 ? 32 : ((192 / (N * N)) < 1 ? 1 : (192 / (N * N)));
+  return N <= 2 ? 32 : ((160 / (N * N)) < 1 ? 1 : (160 / (N * N)));
 }
 template <int N> constexpr int epb2() {
   return (256 / (N * N)) < 1 ? 1 : (256 / (N * N));
@@ -78,207 +98,177 @@ __device__ __forceinline__ void node_geom(const Geom<T> &g, int64_t node, NodeGe
 }
 
 // ---------------------------------------------------------------------
-// 3-d Helmholtz apply: uo = p * sum_k Dk^T M Gk Dk u + q M u
+// Helmholtz apply with a diagonal metric: uo = p sum_k Dk^T M Gk Dk u + q M u,
+// per-node geometry (REGULAR) or per-node p on affine elements.
 // ---------------------------------------------------------------------
 // LD is the input loader (k_maps.cuh): the element-local vector itself, or
 // a unique-node vector gathered through the box lattice or node_class.
 // T is the arithmetic type; the input is stored as LD::value_type and the
 // output as TO (FP32 storage with FP64 arithmetic keeps the apply's
 // rounding at the storage level, which the mixed-precision CG relies on).
+//
+// With a diagonal metric D^T (M G p) D acts along one line, so a line is read
+// once, contracted twice in registers and written once.  The weights M G p are
+// formed by the owner of the node's z-column, which reads the geometry and
+// coefficient planes once and coalesced, and go through shared memory to the
+// x- and y-lines (a line's result then overwrites its weights).  Reading the
+// planes where each direction needs them cost three passes over them, two of
+// them strided: 70 us at 17x22x19 elements, p = 6, FP64 with per-node p and q,
+// against a floor of 23 us for the planes themselves.
+// FP64 holds a line and its contraction in registers and waits on memory and on
+// the line's chain, so small blocks that leave room for many others come first:
+// about 96 threads (N = 4, 5, 6: 33, 43, 54 us against 35, 55, 60 with 160 to
+// 192), one element from N = 7, and the register cap below.  Per-node p and q,
+// 2.4 M nodes (N = 7: cap 64, 72, 80, none: 58, 54, 51, 57 us) and 1.7 M (N = 8:
+// 80, 96, 128, none: 58, 50, 43, 49; a cap that spills loses more than the extra
+// warps give; N = 9: 80, 128, none: 74, 59, 104).
+template <typename T, int N> constexpr int epb_diag() {
+  return sizeof(T) == 4 ? epb3<N>() : (N <= 2 ? 24 : (96 / (N * N) < 1 ? 1 : 96 / (N * N)));
+}
+template <typename T, int N, int EPB> constexpr int helm3_blocks() {
+  constexpr int warps = (N * N * EPB + 31) / 32, regs = N <= 6 ? 56 : (N == 7 ? 80 : 128);
+  return sizeof(T) == 4 ? 0 : 65536 / (warps * 32 * regs);
+}
 template <typename T, int N, int EPB, class LD, typename TO = T>
-__global__ void __launch_bounds__(N *N *EPB)
+__global__ void __launch_bounds__(N *N *EPB, helm3_blocks<T, N, EPB>())
     k_helm3d(const __grid_constant__ Basis<T, N> B, const Geom<T> g, int64_t ne, T p,
              const T *__restrict__ pvec, T q, const T *__restrict__ qvec, int use_mass,
              const LD ld, TO *__restrict__ uo, const double *__restrict__ stop) {
   if (stop && stop[0] != 0.0) return;
   constexpr int P = Pad<N>::P, PLANE = N * P, VOL = N * PLANE, NN = N * N, NNN = N * N * N;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *s = reinterpret_cast<T *>(smem_raw) + threadIdx.y * 3 * VOL;
-  T *su = s, *sgx = s + VOL, *sgy = s + 2 * VOL;
-  const int t = threadIdx.x;
+  T *su = reinterpret_cast<T *>(smem_raw) + threadIdx.y * 5 * VOL;
+  T *sx = su + VOL, *sy = su + 2 * VOL, *sz = su + 3 * VOL, *so = su + 4 * VOL;
+  const int t = threadIdx.x, a0 = t % N, a1 = t / N;
   const int64_t e = (int64_t)blockIdx.x * EPB + threadIdx.y;
   const bool active = e < ne;
-  const int a0 = t % N, a1 = t / N;
   const int64_t base = e * NNN;
+  const int xl = a1 * PLANE + a0 * P, yl = a1 * PLANE + a0, zl = a1 * P + a0;
 
-  NodeGeom<T, 3> eg;
-  eg.X[0] = eg.X[1] = eg.X[2] = eg.J = T(0);
-  if (active) elem_geom<T, 3>(g, e, eg);
-
-  // stage 0: load z-line (i=a0, j=a1) into registers and shared memory
-  T ru[N];
+  // this thread's z-column (i = a0, j = a1): u, the weights, the mass term
   if (active) {
+    NodeGeom<T, 3> eg;
+    eg.X[0] = eg.X[1] = eg.X[2] = eg.J = T(0);
+    elem_geom<T, 3>(g, e, eg);
     typename LD::value_type lv[N];
     ld.template zline<N>(e, a0, a1, lv);
-#pragma unroll
-    for (int k = 0; k < N; k++) ru[k] = (T)lv[k];
-  } else {
-#pragma unroll
-    for (int k = 0; k < N; k++) ru[k] = T(0);
-  }
-#pragma unroll
-  for (int k = 0; k < N; k++) su[k * PLANE + a1 * P + a0] = ru[k];
-  __syncthreads();
-
-  // stage 1: x-line (j=a0, k=a1)
-  {
-    const int j = a0, k = a1;
-    T a[N], d[N];
-#pragma unroll
-    for (int m = 0; m < N; m++) a[m] = su[k * PLANE + j * P + m];
-    line_D<T, N>(B.D, a, d);
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-      NodeGeom<T, 3> ng = eg;
-      const int64_t node = base + k * NN + j * N + i;
-      if (active) node_geom<T, 3>(g, node, ng);
-      T gv = d[i] * (ng.X[0] * ng.X[0]);
-      if (pvec && active) gv *= pvec[node];
-      T mass = B.W[k] * B.W[j] * B.W[i] * ng.J;
-      sgx[k * PLANE + j * P + i] = mass * gv;
-    }
-  }
-  // stage 2: y-line (i=a0, k=a1)
-  {
-    const int i = a0, k = a1;
-    T a[N], d[N];
-#pragma unroll
-    for (int m = 0; m < N; m++) a[m] = su[k * PLANE + m * P + i];
-    line_D<T, N>(B.D, a, d);
-#pragma unroll
-    for (int j = 0; j < N; j++) {
-      NodeGeom<T, 3> ng = eg;
-      const int64_t node = base + k * NN + j * N + i;
-      if (active) node_geom<T, 3>(g, node, ng);
-      T gv = d[j] * (ng.X[1] * ng.X[1]);
-      if (pvec && active) gv *= pvec[node];
-      T mass = B.W[k] * B.W[j] * B.W[i] * ng.J;
-      sgy[k * PLANE + j * P + i] = mass * gv;
-    }
-  }
-  // stage 3: z-line (i=a0, j=a1) in registers
-  T rgz[N];
-  {
-    const int i = a0, j = a1;
-    T d[N];
-    line_D<T, N>(B.D, ru, d);
+    const T w2 = B.W[a0] * B.W[a1];
 #pragma unroll
     for (int k = 0; k < N; k++) {
+      const int64_t node = base + k * NN + t;
+      const int s = zl + k * PLANE;
       NodeGeom<T, 3> ng = eg;
-      const int64_t node = base + k * NN + j * N + i;
-      if (active) node_geom<T, 3>(g, node, ng);
-      T gv = d[k] * (ng.X[2] * ng.X[2]);
-      if (pvec && active) gv *= pvec[node];
-      T mass = B.W[k] * B.W[j] * B.W[i] * ng.J;
-      rgz[k] = mass * gv;
+      node_geom<T, 3>(g, node, ng);
+      const T u = (T)lv[k], mass = B.W[k] * w2 * ng.J;
+      const T mp = pvec ? mass * pvec[node] : mass * p;
+      su[s] = u;
+      sx[s] = mp * (ng.X[0] * ng.X[0]);
+      sy[s] = mp * (ng.X[1] * ng.X[1]);
+      sz[s] = mp * (ng.X[2] * ng.X[2]);
+      so[s] = use_mass ? mass * (qvec ? qvec[node] : q) * u : T(0);
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+      const int s = zl + k * PLANE;
+      su[s] = sx[s] = sy[s] = sz[s] = so[s] = T(0);
     }
   }
   __syncthreads();
-  // stage 4: x-lines of Dx^T, in place
-  {
-    const int j = a0, k = a1;
-    T a[N], d[N];
+  // one line: a = D^T (w (D a))
+  T a[1][N], d[1][N];
+  auto line = [&](const T *w, int s0, int st) {
 #pragma unroll
-    for (int m = 0; m < N; m++) a[m] = sgx[k * PLANE + j * P + m];
-    line_DT<T, N>(B.D, a, d);
+    for (int m = 0; m < N; m++) a[0][m] = su[s0 + m * st];
+    lines_D<T, N, 1, false>(B.D, a, [&](int, int i, T v) { d[0][i] = v * w[s0 + i * st]; });
+    lines_D<T, N, 1, true>(B.D, d, [&](int, int i, T v) { a[0][i] = v; });
+  };
+  line(sx, xl, 1);
 #pragma unroll
-    for (int i = 0; i < N; i++) sgx[k * PLANE + j * P + i] = d[i];
-  }
-  // stage 5: y-lines of Dy^T, in place
-  {
-    const int i = a0, k = a1;
-    T a[N], d[N];
+  for (int m = 0; m < N; m++) sx[xl + m] = a[0][m];
+  line(sy, yl, P);
 #pragma unroll
-    for (int m = 0; m < N; m++) a[m] = sgy[k * PLANE + m * P + i];
-    line_DT<T, N>(B.D, a, d);
-#pragma unroll
-    for (int j = 0; j < N; j++) sgy[k * PLANE + j * P + i] = d[j];
-  }
+  for (int m = 0; m < N; m++) sy[yl + m * P] = a[0][m];
+  line(sz, zl, PLANE);
   __syncthreads();
-  // stage 6: z-lines, combine, mass term, store
-  {
-    const int i = a0, j = a1;
-    T d[N];
-    line_DT<T, N>(B.D, rgz, d);
-    if (active) {
+  if (active) {
 #pragma unroll
-      for (int k = 0; k < N; k++) {
-        const int64_t node = base + k * NN + j * N + i;
-        T o = (sgx[k * PLANE + j * P + i] + sgy[k * PLANE + j * P + i]) + d[k];
-        if (!pvec) o *= p;
-        if (use_mass) {
-          NodeGeom<T, 3> ng = eg;
-          node_geom<T, 3>(g, node, ng);
-          T mu = (B.W[k] * B.W[j] * B.W[i] * ng.J) * ru[k];
-          mu *= qvec ? qvec[node] : q;
-          o += mu;
-        }
-        uo[node] = (TO)o;
-      }
+    for (int k = 0; k < N; k++) {
+      const int s = zl + k * PLANE;
+      uo[base + k * NN + t] = (TO)(((sx[s] + sy[s]) + a[0][k]) + so[s]);
     }
   }
 }
 
-// ---------------------------------------------------------------------
-// 2-d Helmholtz apply (one thread per node)
-// ---------------------------------------------------------------------
+// 2-d: 2 N threads per element, one x-line (threads < N) or y-line each; the
+// block's nodes are loaded and stored by all of its threads, coalesced.  (One
+// thread per node reads D at a run-time row from the parameter bank, which
+// serves one address per cycle: 2 N N-way replays per node.)
+template <int N> constexpr int epb2l() {
+  return (256 / (2 * N)) < 1 ? 1 : 256 / (2 * N);
+}
 template <typename T, int N, int EPB, class LD>
-__global__ void __launch_bounds__(N *N *EPB)
+__global__ void __launch_bounds__(2 * N *EPB)
     k_helm2d(const __grid_constant__ Basis<T, N> B, const Geom<T> g, int64_t ne, T p,
              const T *__restrict__ pvec, T q, const T *__restrict__ qvec, int use_mass,
              const LD ld, T *__restrict__ uo, const double *__restrict__ stop) {
   if (stop && stop[0] != 0.0) return;
-  constexpr int P = Pad<N>::P, AREA = N * P, NN = N * N;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *s = reinterpret_cast<T *>(smem_raw) + threadIdx.y * 3 * AREA;
-  T *su = s, *sgx = s + AREA, *sgy = s + 2 * AREA;
+  constexpr int P = Pad<N>::P, AREA = N * P, NN = N * N, NT = 2 * N * EPB;
+  constexpr int IT = (EPB * NN + NT - 1) / NT;
+  __shared__ T su[EPB * AREA], sx[EPB * AREA], sy[EPB * AREA], sW[N];
+  const int64_t e0 = (int64_t)blockIdx.x * EPB;
+  const int nel = ne - e0 < EPB ? (int)(ne - e0) : EPB;
   const int t = threadIdx.x;
-  const int64_t e = (int64_t)blockIdx.x * EPB + threadIdx.y;
-  const bool active = e < ne;
-  const int i = t % N, j = t / N;
-  const int64_t node = e * NN + t;
-  NodeGeom<T, 2> ng;
-  ng.X[0] = ng.X[1] = ng.J = T(0);
-  T uv = T(0), pv = T(1);
-  if (active) {
+  if (t < N) sW[t] = B.W[t];
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < IT; it++) {
+    const int i = t + it * NT;
+    if (i >= nel * NN) continue;
+    const int el = i / NN, a = i - el * NN, y = a / N, x = a - y * N;
+    const int64_t e = e0 + el, node = e * NN + a;
+    const int s = el * AREA + y * P + x;
+    NodeGeom<T, 2> ng;
     elem_geom<T, 2>(g, e, ng);
     node_geom<T, 2>(g, node, ng);
-    uv = ld.template point2<N>(e, i, j);
-    if (pvec) pv = pvec[node];
+    const T mass = sW[y] * sW[x] * ng.J;
+    const T mp = pvec ? mass * pvec[node] : mass * p;
+    su[s] = (T)ld.template point2<N>(e, x, y);
+    sx[s] = mp * (ng.X[0] * ng.X[0]);
+    sy[s] = mp * (ng.X[1] * ng.X[1]);
   }
-  su[j * P + i] = uv;
   __syncthreads();
-  T dx = B.D[i] * su[j * P];
-  T dy = B.D[j] * su[i];
+  {
+    const int el = t / (2 * N), l = t - el * 2 * N;
+    if (el < nel) {
+      const bool xdir = l < N;
+      const int s0 = el * AREA + (xdir ? l * P : l - N), st = xdir ? 1 : P;
+      T *w = xdir ? sx : sy;
+      T a[N], d[N];
 #pragma unroll
-  for (int m = 1; m < N; m++) {
-    dx = fma(B.D[i + m * N], su[j * P + m], dx);
-    dy = fma(B.D[j + m * N], su[m * P + i], dy);
+      for (int m = 0; m < N; m++) a[m] = su[s0 + m * st];
+      line_D<T, N>(B.D, a, d);
+#pragma unroll
+      for (int m = 0; m < N; m++) d[m] *= w[s0 + m * st];
+      line_DT<T, N>(B.D, d, a);
+#pragma unroll
+      for (int m = 0; m < N; m++) w[s0 + m * st] = a[m];
+    }
   }
-  const T mass = B.W[j] * B.W[i] * ng.J;
-  T gx = dx * (ng.X[0] * ng.X[0]);
-  T gy = dy * (ng.X[1] * ng.X[1]);
-  if (pvec) {
-    gx *= pv;
-    gy *= pv;
-  }
-  sgx[j * P + i] = mass * gx;
-  sgy[j * P + i] = mass * gy;
   __syncthreads();
-  T ox = B.D[i * N] * sgx[j * P];
-  T oy = B.D[j * N] * sgy[i];
 #pragma unroll
-  for (int m = 1; m < N; m++) {
-    ox = fma(B.D[m + i * N], sgx[j * P + m], ox);
-    oy = fma(B.D[m + j * N], sgy[m * P + i], oy);
-  }
-  if (active) {
-    T o = ox + oy;
-    if (!pvec) o *= p;
+  for (int it = 0; it < IT; it++) {
+    const int i = t + it * NT;
+    if (i >= nel * NN) continue;
+    const int el = i / NN, a = i - el * NN, y = a / N, x = a - y * N;
+    const int64_t e = e0 + el, node = e * NN + a;
+    const int s = el * AREA + y * P + x;
+    T o = sx[s] + sy[s];
     if (use_mass) {
-      T mu = mass * uv;
-      mu *= qvec ? qvec[node] : q;
-      o += mu;
+      NodeGeom<T, 2> ng;
+      elem_geom<T, 2>(g, e, ng);
+      node_geom<T, 2>(g, node, ng);
+      o = fma(sW[y] * sW[x] * ng.J * (qvec ? qvec[node] : q), su[s], o);
     }
     uo[node] = o;
   }

@@ -34,9 +34,8 @@ template <typename T, class LD>
 struct DefLaunch {
   template <int N>
   struct F {
-    static int run(gf_problem *prob, int mode, T p, const T *pvec, T q, const T *qvec,
-                   int use_mass, LD ld, int nv, const T *const *c, int idir, T *uo,
-                   cudaStream_t st, const double *stop) {
+    static int run(gf_problem *prob, int mode, T nu, LD ld, int nv, const T *const *c, int idir,
+                   T *uo, cudaStream_t st) {
       const Basis<T, N> B = make_basis<T, N>(prob);
       const DefGeom<T> g = def_of<T>(prob);
       const T *cc[3] = {nullptr, nullptr, nullptr};
@@ -48,15 +47,13 @@ struct DefLaunch {
       if (prob->dim == 3) {
         auto kern = k_def<T, N, 3, LD, T>;
         set_smem(kern, smem);
-        kern<<<(unsigned)prob->ne, threads, smem, st>>>(B, g, prob->ne, mode, p, pvec, q, qvec,
-                                                        use_mass, ld, nv, cc[0], cc[1], cc[2], idir,
-                                                        imass_of<T>(prob), uo, stop);
+        kern<<<(unsigned)prob->ne, threads, smem, st>>>(B, g, prob->ne, mode, nu, ld, nv, cc[0],
+                                                        cc[1], cc[2], idir, imass_of<T>(prob), uo);
       } else {
         auto kern = k_def<T, N, 2, LD, T>;
         set_smem(kern, smem);
-        kern<<<(unsigned)prob->ne, threads, smem, st>>>(B, g, prob->ne, mode, p, pvec, q, qvec,
-                                                        use_mass, ld, nv, cc[0], cc[1], cc[2], idir,
-                                                        imass_of<T>(prob), uo, stop);
+        kern<<<(unsigned)prob->ne, threads, smem, st>>>(B, g, prob->ne, mode, nu, ld, nv, cc[0],
+                                                        cc[1], cc[2], idir, imass_of<T>(prob), uo);
       }
       return GF_OK;
     }
@@ -73,8 +70,22 @@ struct HelmLaunch {
         if constexpr (!std::is_same<T, TO>::value) {
           return GF_ERR_UNSUPPORTED;
         } else {
-          return DefLaunch<T, LD>::template F<N>::run(prob, DEF_HELM, p, pvec, q, qvec, use_mass,
-                                                      ld, 0, nullptr, 0, uo, st, stop);
+          const Basis<T, N> B = make_basis<T, N>(prob);
+          prob->launches++;
+          if (prob->dim == 3) {
+            constexpr int EPB = epb3<N>();
+            const size_t smem = sizeof(T) * 3 * N * N * Pad<N>::P * EPB;
+            auto kern = k_helm3d_full<T, N, EPB, LD>;
+            set_smem(kern, smem);
+            kern<<<(unsigned)((prob->ne + EPB - 1) / EPB), dim3(N * N, EPB), smem, st>>>(
+                B, def_of<T>(prob), prob->ne, p, pvec, q, qvec, use_mass, ld, uo, stop);
+          } else {
+            constexpr int EPB = epb2l<N>();
+            k_helm2d_full<T, N, EPB, LD>
+                <<<(unsigned)((prob->ne + EPB - 1) / EPB), 2 * N * EPB, 0, st>>>(
+                    B, def_of<T>(prob), prob->ne, p, pvec, q, qvec, use_mass, ld, uo, stop);
+          }
+          return GF_OK;
         }
       }
       const Geom<T> g = geom_of<T>(prob);
@@ -107,8 +118,8 @@ struct HelmLaunch {
       }
       const Basis<T, N> B = make_basis<T, N>(prob);
       if (prob->dim == 3) {
-        constexpr int EPB = epb3<N>();
-        const size_t smem = sizeof(T) * 3 * N * N * P * EPB;
+        constexpr int EPB = epb_diag<T, N>();
+        const size_t smem = sizeof(T) * 5 * N * N * P * EPB;
         auto kern = k_helm3d<T, N, EPB, LD, TO>;
         set_smem(kern, smem);
         const unsigned grid = (unsigned)((prob->ne + EPB - 1) / EPB);
@@ -118,14 +129,11 @@ struct HelmLaunch {
       } else if constexpr (!std::is_same<T, TO>::value) {
         return GF_ERR_UNSUPPORTED;  // mixed storage/arithmetic is 3-d only
       } else {
-        constexpr int EPB = epb2<N>();
-        const size_t smem = sizeof(T) * 3 * N * P * EPB;
-        auto kern = k_helm2d<T, N, EPB, LD>;
-        set_smem(kern, smem);
+        constexpr int EPB = epb2l<N>();
         const unsigned grid = (unsigned)((prob->ne + EPB - 1) / EPB);
         prob->launches++;
-        kern<<<grid, dim3(N * N, EPB), smem, st>>>(B, g, prob->ne, p, pvec, q, qvec, use_mass, ld,
-                                                    uo, stop);
+        k_helm2d<T, N, EPB, LD><<<grid, 2 * N * EPB, 0, st>>>(B, g, prob->ne, p, pvec, q, qvec,
+                                                             use_mass, ld, uo, stop);
       }
       return GF_OK;
     }
@@ -182,7 +190,6 @@ inline void launch_dudt_kernel(gf_problem *prob, T nu, const T *const *f, T *con
   }
   const Basis<T, N> B = make_basis<T, N>(prob);
   const Geom<T> g = geom_of<T>(prob);
-  constexpr int P = Pad<N>::P;
   if (prob->dim == 3) {
     constexpr int NF = EQN == GF_EQN_ADVECT ? 4 : (EQN == GF_EQN_BURGERS ? 3 : 1);
     constexpr int EPB = epb_dudt3<N, NF>();
@@ -194,15 +201,13 @@ inline void launch_dudt_kernel(gf_problem *prob, T nu, const T *const *f, T *con
     kern<<<grid, dim3(N * N, EPB), smem, st>>>(B, g, prob->ne, nu, f[0], f[1], f[2], f[3], imass,
                                                 o[0], o[1], o[2], epi);
   } else {
-    constexpr int NF = EQN == GF_EQN_ADVECT ? 3 : (EQN == GF_EQN_BURGERS ? 2 : 1);
-    constexpr int EPB = epb2<N>();
-    const size_t smem = sizeof(T) * (NF + 2) * N * P * EPB;
+    constexpr int EPB = epb2l<N>();
+    const size_t smem = sizeof(T) * dudt2_words<N, EQN>() * EPB;
     auto kern = k_dudt2d<T, N, EPB, EQN, MODE>;
     set_smem(kern, smem);
     const unsigned grid = (unsigned)((prob->ne + EPB - 1) / EPB);
     prob->launches++;
-    kern<<<grid, dim3(N * N, EPB), smem, st>>>(B, g, prob->ne, nu, f[0], f[1], f[2], f[3], imass,
-                                                o[0], o[1], o[2], epi);
+    kern<<<grid, 2 * N * EPB, smem, st>>>(B, g, prob->ne, nu, f[0], f[1], f[2], imass, o[0], o[1]);
   }
 }
 

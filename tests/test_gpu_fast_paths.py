@@ -144,6 +144,58 @@ def test_cluster_cg_outcomes(ctx):
         cg.solve(H, b, prob.zeros(), prob.zeros())
 
 
+@pytest.mark.parametrize("p", ORDERS)
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("geom", ["regular", "deformed", "affine"])
+def test_line_applies(ctx, p, dim, geom):
+    import torch
+    from geoflow_b200 import GHelmholtz, GridBox, Problem
+    ne = [3, 2, 2][:dim]
+    g = GridBox(dim, ne, p)
+    N, n = g.ndof(), p + 1
+    rng = np.random.default_rng(10 * p + dim)
+    shape = [g.nelems] + [n] * dim
+    D, W = g.D.reshape(n, n).T, g.W  # D[l, m]
+    w = W
+    for _ in range(dim - 1):
+        w = np.multiply.outer(W, w)
+    if geom == "deformed":
+        X = rng.standard_normal((dim, dim, N)) * 0.3 + 2.0 * np.eye(dim)[:, :, None]
+        J = 0.1 + rng.random(N)
+        prob = Problem(ctx, g, structured=False, geometry="deformed",
+                       node_geom=np.concatenate([X.reshape(-1), J]))
+    else:
+        prob = Problem(ctx, g, geometry=geom)
+        eg = g.elem_geom.reshape(g.nelems, dim + 1)
+        X = np.zeros((dim, dim, N))
+        for d in range(dim):
+            X[d, d] = np.repeat(eg[:, d], n**dim)
+        J = np.repeat(eg[:, dim], n**dim)
+    u, pv, qv = rng.standard_normal(N), 1.0 + rng.random(N), 1.0 + rng.random(N)
+    mass = w[None] * J.reshape(shape)
+
+    def along(M, f, d):  # contraction along reference direction d (0 = x, the last axis)
+        return np.moveaxis(np.tensordot(M, f, axes=(1, dim - d)), 0, dim - d)
+
+    U = u.reshape(shape)
+    du = [along(D, U, d) for d in range(dim)]
+    phys = [sum(X[i, k].reshape(shape) * du[i] for i in range(dim)) for k in range(dim)]
+    for vec in (False, True):
+        P, Q = (pv.reshape(shape), qv.reshape(shape)) if vec else (0.6, 1.7)
+        ref = Q * mass * U
+        for i in range(dim):
+            flux = P * mass * sum(X[i, k].reshape(shape) * phys[k] for k in range(dim))
+            ref = ref + along(D.T, flux, i)
+        ref = cuda(ref.reshape(-1), torch.float64)
+        for dt, tol in ((torch.float64, 1e-12), (torch.float32, 2e-5)):
+            H = GHelmholtz(prob)
+            H.set_Lap_scalar(cuda(pv, dt) if vec else 0.6)
+            H.set_mass_scalar(cuda(qv, dt) if vec else 1.7)
+            out = prob.zeros(dt)
+            H.opVec_prod(cuda(u, dt), None, out)
+            assert rel(out, ref) < tol, (vec, dt, rel(out, ref))
+
+
 @pytest.mark.parametrize("ne,p", [([33, 31, 33], 2), ([11, 10, 9], 7)])
 def test_multigrid_runs(ctx, ne, p):
     """Multigrid on more than 2^18 points against the Jacobi solve of the same grid
