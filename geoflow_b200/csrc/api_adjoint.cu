@@ -30,6 +30,7 @@
 #include "k_vec.cuh"
 #include "ops_launch.cuh"
 #include "rk_common.cuh"
+#include "rk_pass.cuh"
 
 using namespace gfk;
 
@@ -323,28 +324,10 @@ int vjp(gf_problem *prob, int eqn, double nu, int nstate, const double *const *u
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (n); \
        i += (int64_t)gridDim.x * blockDim.x)
 
-// Butcher reverse, start: acc = lw; lamK_m = cm * lw
-__global__ void k_adj_start(int64_t n, const double *__restrict__ lw, double *__restrict__ acc,
-                            double *K0, double *K1, double *K2, double *K3, double c0, double c1,
-                            double c2, double c3) {
+// out = acc + x on every component
+__global__ void k_adj_add(int64_t n, int nc, RKPass<double> p) {
   GSTRIDE(i, n) {
-    const double v = lw[i];
-    acc[i] = v;
-    K0[i] = c0 * v;
-    if (K1) K1[i] = c1 * v;
-    if (K2) K2[i] = c2 * v;
-    if (K3) K3[i] = c3 * v;
-  }
-}
-// Butcher reverse, stage m: acc += l; lamK_j += b_j l (j < m)
-__global__ void k_adj_fan(int64_t n, const double *__restrict__ l, double *__restrict__ acc,
-                          double *K0, double *K1, double *K2, double b0, double b1, double b2) {
-  GSTRIDE(i, n) {
-    const double v = l[i];
-    acc[i] += v;
-    if (K0) K0[i] += b0 * v;
-    if (K1) K1[i] += b1 * v;
-    if (K2) K2[i] += b2 * v;
+    for (int j = 0; j < nc; j++) p.out[j][i] = p.acc[j][i] + p.x[j][i];
   }
 }
 // SSP reverse, substep m: Sm += a lv + ad f; Sy += b lv; Sy2 += b2 lv
@@ -389,8 +372,9 @@ struct Reverse {
   int64_t n;
   int nstate, ns;
   unsigned g;
-  double *lamK[4][3] = {{nullptr}};  // Butcher: cotangents of K_m; SSP: of stage inputs
-  double *acc[3] = {nullptr}, *tmp[3] = {nullptr};
+  // SSP: cotangents of the stage inputs; Butcher: lamK[0] the smoothed lam
+  double *lamK[4][3] = {{nullptr}};
+  double *acc[3] = {nullptr}, *tmp[3] = {nullptr}, *mu[3] = {nullptr};
   bool ok = true;
 
   Reverse(gf_problem *p, gfrk::Stepper<double> &s, int slot)
@@ -400,13 +384,14 @@ struct Reverse {
       acc[k] = (double *)gf_work(p, slot++, sizeof(double) * n);
       tmp[k] = (double *)gf_work(p, slot++, sizeof(double) * n);
       ok = ok && acc[k] && tmp[k];
-      for (int m = 0; m < ns; m++) {
-        lamK[m][k] = (double *)gf_work(p, slot++, sizeof(double) * n);
-        ok = ok && lamK[m][k];
-      }
+      const bool rk = S.scheme <= 4;
+      if (rk) ok = ok && (mu[k] = (double *)gf_work(p, slot + 4, sizeof(double) * n));
+      for (int m = 0; m < (rk ? 1 : ns); m++)
+        ok = ok && (lamK[m][k] = (double *)gf_work(p, slot + m, sizeof(double) * n));
+      slot += 5;
     }
   }
-  static int slots(int nstate) { return nstate * 6; }
+  static int slots(int nstate) { return nstate * 7; }
   // Smooth (its own transpose) on every state component: one lattice pass
   // on box problems (the stepper's multi-component kernel), CSR otherwise
   void smooth_n(double *const *v) { S.smooth_n(v); }
@@ -418,33 +403,38 @@ struct Reverse {
   }
 
   // uout = S(uin + sum_m c_m h K_m), K_m = S F(u^m),
-  // u^m = uin + sum_{j<m} beta_mj h K_j (m < ns-1), u^{ns-1} = S(same).
+  // u^m = uin + beta_m,m-1 h K_m-1 (m < ns-1), u^{ns-1} = S(same); every tableau
+  // here has one term per stage, so the reverse is one pass per stage:
+  //   start:    L = S lam;  acc = L;  mu = c_{ns-1} h L  (the last stage's cotangent)
+  //   stage m:  t = F'(u^m)^T mu;  acc += t (S t for the last stage, whose input
+  //             is smoothed);  mu = c_{m-1} h L + beta_m,m-1 h S t
+  // S is idempotent, so mu, the Smooth of c h L + beta h t, needs no other pass.
   int butcher(double *const *tape, double *const *lam, double h) {
     double alpha[4], beta[4][4], cc[4];
     gfrk::butcher(S.scheme, alpha, beta, cc);
-    smooth_n(lam);
+    RKPass<double> p{};
     for (int k = 0; k < nstate; k++) {
-      prob->launches++;
-      k_adj_start<<<g, 256, 0, st>>>(n, lam[k], acc[k], lamK[0][k], ns > 1 ? lamK[1][k] : nullptr,
-                                     ns > 2 ? lamK[2][k] : nullptr, ns > 3 ? lamK[3][k] : nullptr,
-                                     cc[0] * h, cc[1] * h, cc[2] * h, cc[3] * h);
+      p.x[k] = lam[k];
+      p.acc[k] = acc[k];
+      p.aux[k] = lamK[0][k];
+      p.out[k] = mu[k];
     }
+    p.ch = cc[ns - 1] * h;
+    rk_pass<double>(prob, ADJ_START, nstate, p, st);
+    for (int k = 0; k < nstate; k++) p.x[k] = tmp[k];
     for (int m = ns - 1; m >= 0; m--) {
-      double *mu[3] = {lamK[m][0], lamK[m][1], lamK[m][2]};
-      smooth_n(mu);
       const double *um[3] = {tape[3 * m], tape[3 * m + 1], tape[3 * m + 2]};
       int rc = vjp(prob, S.eqn, (double)S.nu, nstate, um, S.c, (const double *const *)mu, tmp);
       if (rc) return rc;
-      if (m == ns - 1) smooth_n(tmp);
-      for (int k = 0; k < nstate; k++) {
-        prob->launches++;
-        k_adj_fan<<<g, 256, 0, st>>>(n, tmp[k], acc[k], m > 0 ? lamK[0][k] : nullptr,
-                                     m > 1 ? lamK[1][k] : nullptr, m > 2 ? lamK[2][k] : nullptr,
-                                     beta[m][0] * h, beta[m][1] * h, beta[m][2] * h);
-      }
+      if (m == 0) break;
+      p.ch = cc[m - 1] * h;
+      p.b = beta[m][m - 1] * h;
+      rk_pass<double>(prob, m == ns - 1 ? ADJ_STAGE_LAST : ADJ_STAGE, nstate, p, st);
     }
-    for (int k = 0; k < nstate; k++)
-      cudaMemcpyAsync(lam[k], acc[k], sizeof(double) * n, cudaMemcpyDeviceToDevice, st);
+    if (ns == 1) smooth_n(tmp);
+    for (int k = 0; k < nstate; k++) p.out[k] = lam[k];
+    prob->launches++;
+    k_adj_add<<<g, 256, 0, st>>>(n, nstate, p);
     return GF_OK;
   }
 
@@ -620,15 +610,27 @@ extern "C" int gf_adjoint_gradient(gf_problem_t prob, const gf_rk_traits *traits
   auto d2d = [&](double *dst, const double *src) {
     cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, st);
   };
+  // steps s0 .. s1-1 from the state in ua, whose result ends in ua; with the
+  // tape on, each state is written where the tape keeps it
+  auto segment = [&](int s0, int s1, bool taped) -> int {
+    if (taped)
+      for (int k = 0; k < nst; k++) d2d(tp(0)[k], ua[k]);
+    for (int s = s0; s < s1; s++) {
+      double *const *in = taped ? tp(s - s0) : ua;
+      const bool last = s + 1 == s1;
+      double *const *out = taped && !last ? tp(s - s0 + 1) : ub;
+      int r = S.step(in, out, dt, taped ? tp(s - s0) : nullptr);
+      if (r) return r;
+      if (!taped || last) std::swap(ua, ub);
+    }
+    return GF_OK;
+  };
   // forward sweep; the last segment is taped on the way
   for (int k = 0; k < nst; k++) d2d(ua[k], u0[k]);
-  const int last0 = nseg > 0 ? (nseg - 1) * C : 0;
-  for (int s = 0; s < nsteps; s++) {
-    if (s % C == 0)
-      for (int k = 0; k < nst; k++) d2d(ck[(s / C) * 3 + k], ua[k]);
-    if ((rc = S.step(ua, ub, dt, s >= last0 ? tp(s - last0) : nullptr)))
+  for (int sg = 0; sg < nseg; sg++) {
+    for (int k = 0; k < nst; k++) d2d(ck[sg * 3 + k], ua[k]);
+    if ((rc = segment(sg * C, std::min(nsteps, (sg + 1) * C), sg == nseg - 1)))
       return gf_fail(ctx, rc, "forward step failed");
-    std::swap(ua, ub);
   }
   // J and its gradient with respect to u(T): lam = M (u(T) - obs)
   double *Jd = prob->scal_d + 60;
@@ -643,10 +645,7 @@ extern "C" int gf_adjoint_gradient(gf_problem_t prob, const gf_rk_traits *traits
     const int s0 = sg * C, s1 = std::min(nsteps, s0 + C);
     if (sg != nseg - 1) {  // recompute the segment with the tape on
       for (int k = 0; k < nst; k++) d2d(ua[k], ck[sg * 3 + k]);
-      for (int s = s0; s < s1; s++) {
-        if ((rc = S.step(ua, ub, dt, tp(s - s0)))) return gf_fail(ctx, rc, "recompute failed");
-        std::swap(ua, ub);
-      }
+      if ((rc = segment(s0, s1, true))) return gf_fail(ctx, rc, "recompute failed");
     }
     for (int s = s1 - 1; s >= s0; s--)
       if ((rc = R.run(tp(s - s0), grad, dt))) return gf_fail(ctx, rc, "reverse step failed");

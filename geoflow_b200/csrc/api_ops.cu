@@ -298,22 +298,44 @@ extern "C" int gf_dudt(gf_problem_t prob, int dtype, int eqn, double nu, int nst
 // gather-scatter
 // ---------------------------------------------------------------------
 template <typename T>
+struct DssBoxLaunch {
+  template <int N>
+  struct F {
+    static int run(gf_problem *prob, int op, T *u, cudaStream_t st) {
+      const RunWalk<N - 1> w = RunWalk<N - 1>::make(prob->box);
+      const RunGrid g = run_grid(prob, w);
+      prob->launches++;
+      switch (op) {
+        case GF_DSS_SUM: k_dss_box<T, GF_DSS_SUM, N - 1><<<g.blocks, g.block, 0, st>>>(u, w, g); break;
+        case GF_DSS_SMOOTH: k_dss_box<T, GF_DSS_SMOOTH, N - 1><<<g.blocks, g.block, 0, st>>>(u, w, g); break;
+        case GF_DSS_MAX: k_dss_box<T, GF_DSS_MAX, N - 1><<<g.blocks, g.block, 0, st>>>(u, w, g); break;
+        case GF_DSS_MIN: k_dss_box<T, GF_DSS_MIN, N - 1><<<g.blocks, g.block, 0, st>>>(u, w, g); break;
+        default: prob->launches--; return GF_ERR_ARG;
+      }
+      return GF_OK;
+    }
+  };
+};
+
+template <typename T>
 int launch_dss(gf_problem *prob, int op, T *u, cudaStream_t st) {
-  unsigned grid = grid_for(prob->nclass, 256, prob->ctx->sm_count * 16);
   BoxWalk w;
-  if (dss_box_walk(prob, w)) {  // lattice classes: no index arrays
+  const bool box = dss_box_walk(prob, w);  // lattice classes: no index arrays
+  if (box && w.nL < POINT_NODES) {
+    const unsigned grid = grid_for(w.nL, 256, prob->ctx->sm_count * 16);
     prob->launches++;
     switch (op) {
-      case GF_DSS_SUM: k_dss_box<T, GF_DSS_SUM><<<grid, 256, 0, st>>>(u, w); break;
-      case GF_DSS_SMOOTH: k_dss_box<T, GF_DSS_SMOOTH><<<grid, 256, 0, st>>>(u, w); break;
-      case GF_DSS_MAX: k_dss_box<T, GF_DSS_MAX><<<grid, 256, 0, st>>>(u, w); break;
-      case GF_DSS_MIN: k_dss_box<T, GF_DSS_MIN><<<grid, 256, 0, st>>>(u, w); break;
+      case GF_DSS_SUM: k_dss_point<T, GF_DSS_SUM><<<grid, 256, 0, st>>>(u, w); break;
+      case GF_DSS_SMOOTH: k_dss_point<T, GF_DSS_SMOOTH><<<grid, 256, 0, st>>>(u, w); break;
+      case GF_DSS_MAX: k_dss_point<T, GF_DSS_MAX><<<grid, 256, 0, st>>>(u, w); break;
+      case GF_DSS_MIN: k_dss_point<T, GF_DSS_MIN><<<grid, 256, 0, st>>>(u, w); break;
       default: prob->launches--; return GF_ERR_ARG;
     }
     return GF_OK;
   }
+  if (box) return dispatch_n<DssBoxLaunch<T>::template F>(prob->n, prob, op, u, st);
   const SplitCls sc = split_of(prob);
-  grid = grid_for(sc.n + sc.nsh, 256, prob->ctx->sm_count * 16);
+  const unsigned grid = grid_for(sc.n + sc.nsh, 256, prob->ctx->sm_count * 16);
   prob->launches++;
   switch (op) {
     case GF_DSS_SUM: k_dss_split<T, GF_DSS_SUM><<<grid, 256, 0, st>>>(u, sc); break;

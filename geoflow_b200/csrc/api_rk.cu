@@ -4,10 +4,12 @@
 //   Butcher step_b (1)  (gexrk_stepper.ipp:252-341), tableau of
 //                       GButcherRK::computeCoeffs (gbutcherrk.ipp:69-125)
 //   SSP22 / SSP33 / SSP34 (gexrk_stepper.ipp:533-780), step_euler (809-819)
-// and GBurgers::step_impl (gburgers.ipp:275-333): uold = u; step(uold -> u).
+// and GBurgers::step_impl (gburgers.ipp:275-333).
 //
-// Per stage: one fused element kernel for the RHS (k_dudt*), one class
-// kernel for Smooth, and elementwise stage combinations.
+// Per stage: the fused element kernel of the RHS (k_dudt*) and one class pass
+// (rk_pass.cuh) that smooths its result and forms the next stage's input and the
+// running sum; the step reads its input state and writes the result, in place
+// where they are the same.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -17,12 +19,13 @@
 #include "k_vec.cuh"
 #include "ops_launch.cuh"
 #include "rk_common.cuh"
+#include "rk_pass.cuh"
 
 using namespace gfk;
 
 namespace gfrk {
 
-// slot of the problem's scalar block holding the RK non-finite flag
+// slot of the problem's host scalar block holding the RK non-finite flag
 constexpr int RK_FLAG_SLOT = 62;
 
 void butcher(int order, double *alpha, double beta[4][4], double *c) {
@@ -69,17 +72,31 @@ __global__ void k_stage_sum(int64_t n, const T *__restrict__ uin, int nk, const 
 
 // flag[0] = 1 when any of the nstate fields holds a non-finite value
 // (GBurgers::step_impl asserts isfinite on the evolved state after every
-// step, gburgers.ipp:325-331).  Only a bad value writes the flag.
+// step, gburgers.ipp:325-331).  Only a bad value writes the flag.  16-byte
+// loads where the field is aligned to them, several in flight per thread
+// (scalar: 59 us for three FP32 fields of 13.8 M values, 25 at HBM rate).
 template <typename T>
-__global__ void k_nonfinite(int64_t n, int nstate, const T *__restrict__ u0,
-                            const T *__restrict__ u1, const T *__restrict__ u2,
-                            double *__restrict__ flag) {
+__global__ void __launch_bounds__(256)
+    k_nonfinite(int64_t n, int nstate, const T *u0, const T *u1, const T *u2, double *flag) {
+  constexpr int V = 16 / sizeof(T);
+  struct alignas(16) Vec {
+    T v[V];
+  };
+  const T *const u[3] = {u0, u1, u2};
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   bool bad = false;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    bad |= !isfinite(u0[i]);
-    if (nstate > 1) bad |= !isfinite(u1[i]);
-    if (nstate > 2) bad |= !isfinite(u2[i]);
+#pragma unroll
+  for (int f = 0; f < 3; f++) {
+    if (f >= nstate) break;
+    const int64_t nv = reinterpret_cast<uintptr_t>(u[f]) % 16 == 0 ? n / V : 0;
+#pragma unroll 4
+    for (int64_t i = t0; i < nv; i += stride) {
+      const Vec q = reinterpret_cast<const Vec *>(u[f])[i];
+#pragma unroll
+      for (int k = 0; k < V; k++) bad |= !isfinite(q.v[k]);
+    }
+    for (int64_t i = nv * V + t0; i < n; i += stride) bad |= !isfinite(u[f][i]);
   }
   if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) flag[0] = 1.0;
 }
@@ -203,7 +220,7 @@ bool Stepper<T>::rhs_euler_smooth(T *const *u, T *const *x, T dt, T *const *uin,
   if (eqn == GF_EQN_HEAT) {
     for (int k = 0; k < nstate; k++) {
       const T *fk[4] = {u[k], nullptr, nullptr, nullptr};
-      T *ok[3] = {x[k], nullptr, nullptr};
+      T *ok[3] = {utmp[k], nullptr, nullptr};
       const RKEpi<T> e = epi_for(k, 1);
       if ((*rc = launch_dudt<T>(prob, eqn, MODE_EULER, nu, fk, ok, st, &e))) return true;
     }
@@ -211,132 +228,80 @@ bool Stepper<T>::rhs_euler_smooth(T *const *u, T *const *x, T dt, T *const *uin,
     if (eqn == GF_EQN_ADVECT) {
       f[0] = u[0];
       for (int k = 0; k < gf_nvel(prob); k++) f[1 + k] = c[k];
-      o[0] = x[0];
+      o[0] = utmp[0];
     } else {
       for (int k = 0; k < gf_nvel(prob); k++) {
         f[k] = u[k];
-        o[k] = x[k];
+        o[k] = utmp[k];
       }
     }
     const RKEpi<T> e = epi_for(0, nstate);
     if ((*rc = launch_dudt<T>(prob, eqn, MODE_EULER, nu, f, o, st, &e))) return true;
   }
-  smooth_n(x);
+  smooth_to(utmp, x);
   *rc = GF_OK;
   return true;
 }
 
-template <typename T>
-void Stepper<T>::smooth(T *v) {
-  launch_dss<T>(prob, GF_DSS_SMOOTH, v, st);
-}
-
-// gather-scatter Smooth fused with the stage update around it, one
-// component, CSR members (k_dss.cuh); box problems take the *_n forms below
-template <typename T>
-void Stepper<T>::euler_smooth(T *x, T dt, const T *uin, T a, const T *y, T b, T a2, const T *y2,
-                              T b2) {
-  prob->launches++;
-  const SplitCls sc = split_of(prob);
-  k_dss_rk_split<T, FUSE_EULER><<<grid_for(sc.n + sc.nsh, 256, prob->ctx->sm_count * 16), 256, 0,
-                                  st>>>(x, sc, dt, uin, a, y, b, a2, y2, b2, nullptr, nullptr, T(0));
-}
-
-template <typename T>
-void Stepper<T>::smooth_accum(T *K, T ch, T *uout) {
-  prob->launches++;
-  const SplitCls sc = split_of(prob);
-  k_dss_rk_split<T, FUSE_ACCUM_AFTER><<<grid_for(sc.n + sc.nsh, 256, prob->ctx->sm_count * 16), 256,
-                                        0, st>>>(K, sc, T(0), nullptr, T(0), nullptr, T(0), T(0),
-                                                 nullptr, T(0), uout, nullptr, ch);
-}
-
-template <typename T>
-void Stepper<T>::accum_smooth(T *uout, const T *K, T ch) {
-  prob->launches++;
-  const SplitCls sc = split_of(prob);
-  k_dss_rk_split<T, FUSE_ACCUM_BEFORE><<<grid_for(sc.n + sc.nsh, 256, prob->ctx->sm_count * 16),
-                                         256, 0, st>>>(uout, sc, T(0), nullptr, T(0), nullptr, T(0),
-                                                       T(0), nullptr, T(0), nullptr, K, ch);
-}
-
-// Launch k_dss_rk_box_n / k_dss_smooth_box_n for nstate components; false
-// when the problem takes the per-component CSR kernels.
-template <typename T, int MODE>
-static bool launch_rk_n(gf_problem *prob, cudaStream_t st, int nstate, const RKComps<T> &pc,
-                        T dt, T a, T b, T a2, T b2, T ch, bool plain) {
-  BoxWalk w;
-  if (!dss_box_walk(prob, w) || nstate < 1 || nstate > 3) return false;
-  const unsigned grid = grid_for(prob->nclass, 256, prob->ctx->sm_count * 16);
-  prob->launches++;
-  if (plain) {
-    if (nstate == 1) k_dss_smooth_box_n<T, 1><<<grid, 256, 0, st>>>(pc, w);
-    else if (nstate == 2) k_dss_smooth_box_n<T, 2><<<grid, 256, 0, st>>>(pc, w);
-    else k_dss_smooth_box_n<T, 3><<<grid, 256, 0, st>>>(pc, w);
-  } else {
-    if (nstate == 1) k_dss_rk_box_n<T, MODE, 1><<<grid, 256, 0, st>>>(pc, w, dt, a, b, a2, b2, ch);
-    else if (nstate == 2) k_dss_rk_box_n<T, MODE, 2><<<grid, 256, 0, st>>>(pc, w, dt, a, b, a2, b2, ch);
-    else k_dss_rk_box_n<T, MODE, 3><<<grid, 256, 0, st>>>(pc, w, dt, a, b, a2, b2, ch);
-  }
-  return true;
-}
-
-template <typename T>
-static RKComps<T> comps(int nstate, T *const *x, T *const *uin, T *const *y, T *const *y2,
-                        T *const *K, T *const *acc) {
-  RKComps<T> pc{};
-  for (int k = 0; k < nstate && k < 3; k++) {
-    pc.x[k] = x[k];
-    pc.uin[k] = uin ? uin[k] : nullptr;
-    pc.y[k] = y ? y[k] : nullptr;
-    pc.y2[k] = y2 ? y2[k] : nullptr;
-    pc.K[k] = K ? K[k] : nullptr;
-    pc.acc[k] = acc ? acc[k] : nullptr;
-  }
-  return pc;
-}
-
+// v <- Smooth(v) in place
 template <typename T>
 void Stepper<T>::smooth_n(T *const *v) {
-  if (launch_rk_n<T, FUSE_EULER>(prob, st, nstate,
-                                 comps<T>(nstate, v, nullptr, nullptr, nullptr, nullptr, nullptr),
-                                 T(0), T(0), T(0), T(0), T(0), T(0), true))
-    return;
-  for (int k = 0; k < nstate; k++) smooth(v[k]);
+  smooth_to(v, v);
 }
 
 template <typename T>
-void Stepper<T>::euler_smooth_n(T *const *x, T dt, T *const *uin, T a, T *const *y, T b, T a2,
-                                T *const *y2, T b2) {
-  if (launch_rk_n<T, FUSE_EULER>(prob, st, nstate,
-                                 comps<T>(nstate, x, uin, y, y2, nullptr, nullptr), dt, a, b, a2,
-                                 b2, T(0), false))
-    return;
-  for (int k = 0; k < nstate; k++)
-    euler_smooth(x[k], dt, uin[k], a, y ? y[k] : nullptr, b, a2, y2 ? y2[k] : nullptr, b2);
+void Stepper<T>::smooth_to(T *const *v, T *const *out) {
+  RKPass<T> p{};
+  for (int k = 0; k < nstate; k++) {
+    p.x[k] = v[k];
+    p.out[k] = out[k];
+  }
+  rk_pass<T>(prob, RK_SMOOTH, nstate, p, st);
 }
 
 template <typename T>
-void Stepper<T>::smooth_accum_n(T *const *Kv, T ch, T *const *uout) {
-  if (launch_rk_n<T, FUSE_ACCUM_AFTER>(
-          prob, st, nstate, comps<T>(nstate, Kv, nullptr, nullptr, nullptr, nullptr, uout), T(0),
-          T(0), T(0), T(0), T(0), ch, false))
-    return;
-  for (int k = 0; k < nstate; k++) smooth_accum(Kv[k], ch, uout[k]);
+void Stepper<T>::euler_smooth_n(T *const *x, T *const *out, T dt, T *const *uin, T a, T *const *y,
+                                T b, T a2, T *const *y2, T b2) {
+  RKPass<T> p{};
+  for (int k = 0; k < nstate; k++) {
+    p.x[k] = x[k];
+    p.out[k] = out[k];
+    p.uin[k] = uin[k];
+    p.y[k] = y ? y[k] : nullptr;
+    p.y2[k] = y2 ? y2[k] : nullptr;
+  }
+  p.dt = dt;
+  p.a = a;
+  p.b = b;
+  p.a2 = a2;
+  p.b2 = b2;
+  rk_pass<T>(prob, RK_EULER, nstate, p, st);
 }
 
 template <typename T>
-void Stepper<T>::accum_smooth_n(T *const *uout, T *const *Kv, T ch) {
-  if (launch_rk_n<T, FUSE_ACCUM_BEFORE>(
-          prob, st, nstate, comps<T>(nstate, uout, nullptr, nullptr, nullptr, Kv, nullptr), T(0),
-          T(0), T(0), T(0), T(0), ch, false))
-    return;
-  for (int k = 0; k < nstate; k++) accum_smooth(uout[k], Kv[k], ch);
+void Stepper<T>::stage_pass(int mode, T *const *x, T *const *accin, T ch, T *const *accout,
+                            T *const *uin, T b, T *const *out) {
+  RKPass<T> p{};
+  for (int k = 0; k < nstate; k++) {
+    p.x[k] = x[k];
+    p.accin[k] = accin[k];
+    p.acc[k] = accout ? accout[k] : nullptr;
+    p.uin[k] = uin ? uin[k] : nullptr;
+    p.out[k] = out[k];
+  }
+  p.ch = ch;
+  p.b = b;
+  rk_pass<T>(prob, mode, nstate, p, st);
+}
+
+template <typename T>
+bool Stepper<T>::constrains() const {
+  return prob->geom == GF_GEOM_EMBEDDED && nstate >= 3 && prob->xyz_d;
 }
 
 template <typename T>
 void Stepper<T>::constrain(T *const *u) {
-  if (prob->geom != GF_GEOM_EMBEDDED || nstate < 3 || !prob->xyz_d) return;
+  if (!constrains()) return;
   const T *x = sizeof(T) == 8 ? (const T *)prob->xyz_d : (const T *)prob->xyz_f;
   const unsigned g = grid_for(n, 256, prob->ctx->sm_count * 8);
   prob->launches++;
@@ -347,11 +312,15 @@ template <typename T>
 bool Stepper<T>::alloc() {
   const size_t bytes = sizeof(T) * n;
   int slot = 30 + (sizeof(T) == 8 ? 0 : 20);
-  for (int k = 0; k < nstate; k++) {
-    uold[k] = (T *)gf_work(prob, slot++, bytes);
-    utmp[k] = (T *)gf_work(prob, slot++, bytes);
-    for (int j = 0; j < 3; j++) K[j][k] = (T *)gf_work(prob, slot++, bytes);
-    if (!uold[k] || !utmp[k] || !K[0][k] || !K[1][k] || !K[2][k]) return false;
+  // step_b keeps one slope (its accumulated state in uacc); the SSP schemes
+  // the results of all substeps but the last
+  const int nK = scheme <= 4 ? 1 : stages() - 1;
+  for (int k = 0; k < nstate; k++, slot += 5) {
+    uacc[k] = (T *)gf_work(prob, slot, bytes);
+    utmp[k] = (T *)gf_work(prob, slot + 1, bytes);
+    if (!uacc[k] || !utmp[k]) return false;
+    for (int j = 0; j < nK; j++)
+      if (!(K[j][k] = (T *)gf_work(prob, slot + 2 + j, bytes))) return false;
   }
   if (adv_ok()) {
     const int s2 = sizeof(T) == 8 ? 70 : 72;
@@ -362,59 +331,50 @@ bool Stepper<T>::alloc() {
   return true;
 }
 
-// One step uin -> uout (uout may not alias uin).
+// One step uin -> uout (which may be uin).
 template <typename T>
 int Stepper<T>::step(T *const *uin, T *const *uout, T dt, T *const *tape) {
-  const unsigned g = grid_for(n, 256, prob->ctx->sm_count * 8);
   int rc;
+  auto copy = [&](T *const *dst, T *const *src) {  // a caller's tape may hold uin already
+    for (int k = 0; k < nstate; k++)
+      if (dst[k] != src[k])
+        cudaMemcpyAsync(dst[k], src[k], sizeof(T) * n, cudaMemcpyDeviceToDevice, st);
+  };
   if (scheme >= 1 && scheme <= 4) {
     double alpha[4], beta[4][4], cc[4];
     butcher(scheme, alpha, beta, cc);
     const int ns = scheme;
     const T h = dt;
-    // stage inputs go to the tape when one is given
+    // stage inputs go to the tape when one is given; stage 0's is uin itself
     auto stage_in = [&](int m) { return tape ? tape + 3 * m : (T *const *)utmp; };
-    for (int k = 0; k < nstate; k++)
-      cudaMemcpyAsync(uout[k], uin[k], sizeof(T) * n, cudaMemcpyDeviceToDevice, st);
-    for (int m = 0; m < ns - 1; m++) {
-      T *const *um = stage_in(m);
-      for (int k = 0; k < nstate; k++) {
-        prob->launches++;
-        k_stage_sum<T><<<g, 256, 0, st>>>(n, uin[k], m, K[0][k], K[1][k], K[2][k],
-                                          (T)beta[m][0] * h, (T)beta[m][1] * h,
-                                          (T)beta[m][2] * h, um[k]);
-      }
+    T *const *um = uin, *const *acc = uin;
+    if (ns == 1 || tape || constrains()) {
+      um = stage_in(0);
+      if (ns == 1 && um[0] == uin[0]) copy(acc = utmp, uin);  // smoothed in place below
+      copy(um, uin);
+      if (ns == 1) smooth_n(um);
       constrain(um);
-      if ((rc = rhs(um, K[m]))) return rc;
-      smooth_accum_n(K[m], (T)cc[m] * h, uout);
-      constrain(uout);
     }
-    T *const *uf = stage_in(ns - 1);
-    for (int k = 0; k < nstate; k++) {
-      prob->launches++;
-      k_stage_sum<T><<<g, 256, 0, st>>>(n, uin[k], ns - 1, K[0][k], K[1][k], K[2][k],
-                                        (T)beta[ns - 1][0] * h, (T)beta[ns - 1][1] * h,
-                                        (T)beta[ns - 1][2] * h, uf[k]);
+    for (int m = 0; m < ns - 1; m++) {
+      if ((rc = rhs(um, K[0]))) return rc;
+      // the tableaux here have one term per stage: beta[m+1][m]
+      um = stage_in(m + 1);
+      stage_pass(m == ns - 2 ? RK_MIDS : RK_MID, K[0], acc, (T)cc[m] * h, uacc, uin,
+                 (T)beta[m + 1][m] * h, um);
+      acc = uacc;
+      constrain(um);
+      constrain(uacc);
     }
-    smooth_n(uf);
-    constrain(uf);
-    // the final stage result goes to the last K slot (K[0] in the
-    // reference, whose earlier content is no longer needed)
-    T *const *Kf = K[0];
-    if ((rc = rhs(uf, Kf))) return rc;
-    smooth_n(Kf);
-    accum_smooth_n(uout, Kf, (T)cc[ns - 1] * h);
+    if ((rc = rhs(um, K[0]))) return rc;
+    stage_pass(RK_LAST, K[0], acc, (T)cc[ns - 1] * h, nullptr, nullptr, T(0), uout);
     constrain(uout);
     return GF_OK;
   }
   // SSP stage inputs are uin and the substep results left in K[0..ns-2]
   if (tape) {
     if ((rc = step_ssp(uin, uout, dt))) return rc;
-    for (int k = 0; k < nstate; k++) {
-      cudaMemcpyAsync(tape[k], uin[k], sizeof(T) * n, cudaMemcpyDeviceToDevice, st);
-      for (int m = 1; m < stages(); m++)
-        cudaMemcpyAsync(tape[3 * m + k], K[m - 1][k], sizeof(T) * n, cudaMemcpyDeviceToDevice, st);
-    }
+    copy(tape, uin);
+    for (int m = 1; m < stages(); m++) copy(tape + 3 * m, K[m - 1]);
     return GF_OK;
   }
   return step_ssp(uin, uout, dt);
@@ -422,47 +382,52 @@ int Stepper<T>::step(T *const *uin, T *const *uout, T dt, T *const *tape) {
 
 // One SSP substep: x = Smooth(update(dudt(u))), as the RHS call followed by
 // euler_smooth_n, or in two passes (the RHS kernel writing the update,
-// then the Smooth) where the RHS kernel has the fused epilogue.
+// then the Smooth) where the RHS kernel has the fused epilogue.  x may be y
+// or y2 (a step in place): both forms read a node's or class's y before they
+// write it.
 template <typename T>
 static int ssp_substep(Stepper<T> &S, T *const *u, T *const *x, T dt, T *const *uin, T a,
                        T *const *y, T b, T a2, T *const *y2, T b2) {
   int rc = GF_OK;
   if (S.rhs_euler_smooth(u, x, dt, uin, a, y, b, a2, y2, b2, &rc)) return rc;
-  if ((rc = S.rhs(u, x))) return rc;
-  S.euler_smooth_n(x, dt, uin, a, y, b, a2, y2, b2);
+  if ((rc = S.rhs(u, S.utmp))) return rc;
+  S.euler_smooth_n(S.utmp, x, dt, uin, a, y, b, a2, y2, b2);
   return GF_OK;
+}
+
+// Substep m of the SSP schemes (gexrk_stepper.ipp:533-780): from stage input
+// s_m to s_{m+1} = Smooth(a (dt dudt(s_m) + s_m) + b s_y + b2 s_y2), s_0 the
+// step's input (y or y2 -1: no such term).
+template <typename T>
+struct SSPSubstep {
+  T a, b, b2;
+  int y, y2;
+};
+template <typename T>
+static SSPSubstep<T> ssp_coeffs(int scheme, int m) {
+  const T h = T(0.5);
+  if (scheme == GF_SSP22 && m == 1) return {h, h, T(0), 0, -1};
+  if (scheme == GF_SSP33 && m == 1) return {T(0.25), T(0.75), T(0), 0, -1};
+  if (scheme == GF_SSP33 && m == 2) return {T(2.0 / 3.0), T(1.0 / 3.0), T(0), 0, -1};
+  if (scheme == GF_SSP34) {
+    if (m == 2) return {T(1.0 / 6.0), T(1.0 / 6.0), T(2.0 / 3.0), 2, 0};
+    return {h, h, T(0), m, -1};
+  }
+  return {T(1), T(0), T(0), -1, -1};
 }
 
 template <typename T>
 int Stepper<T>::step_ssp(T *const *uin, T *const *uout, T dt) {
-  int rc;
-  const T one = T(1);
-  if (scheme == GF_SSP22) {
-    if ((rc = ssp_substep<T>(*this, uin, K[0], dt, uin, one, nullptr, T(0), one, nullptr, T(0))))
-      return rc;
-    return ssp_substep<T>(*this, K[0], uout, dt, K[0], T(0.5), uin, T(0.5), one, nullptr, T(0));
+  const int ns = stages();
+  auto state = [&](int i) -> T *const * { return i == 0 ? uin : K[i - 1]; };
+  for (int m = 0; m < ns; m++) {
+    const SSPSubstep<T> q = ssp_coeffs<T>(scheme, m);
+    int rc = ssp_substep<T>(*this, state(m), m + 1 < ns ? (T *const *)K[m] : uout, dt, state(m), q.a,
+                            q.y >= 0 ? state(q.y) : nullptr, q.b, T(1),
+                            q.y2 >= 0 ? state(q.y2) : nullptr, q.b2);
+    if (rc) return rc;
   }
-  if (scheme == GF_SSP33) {
-    if ((rc = ssp_substep<T>(*this, uin, K[0], dt, uin, one, nullptr, T(0), one, nullptr, T(0))))
-      return rc;
-    if ((rc = ssp_substep<T>(*this, K[0], K[1], dt, K[0], T(0.25), uin, T(0.75), one, nullptr,
-                             T(0))))
-      return rc;
-    return ssp_substep<T>(*this, K[1], uout, dt, K[1], T(2.0 / 3.0), uin, T(1.0 / 3.0), one,
-                          nullptr, T(0));
-  }
-  if (scheme == GF_SSP34) {
-    if ((rc = ssp_substep<T>(*this, uin, K[0], dt, uin, T(0.5), uin, T(0.5), one, nullptr, T(0))))
-      return rc;
-    if ((rc = ssp_substep<T>(*this, K[0], K[1], dt, K[0], T(0.5), K[0], T(0.5), one, nullptr,
-                             T(0))))
-      return rc;
-    if ((rc = ssp_substep<T>(*this, K[1], K[2], dt, K[1], T(1.0 / 6.0), K[1], T(1.0 / 6.0), one,
-                             uin, T(2.0 / 3.0))))
-      return rc;
-    return ssp_substep<T>(*this, K[2], uout, dt, K[2], T(0.5), K[2], T(0.5), one, nullptr, T(0));
-  }
-  return GF_ERR_ARG;
+  return GF_OK;
 }
 
 template struct Stepper<double>;
@@ -499,9 +464,7 @@ int advance(gf_problem *prob, const gf_rk_traits *tr, void *const *u, const void
   T *uu[3] = {nullptr, nullptr, nullptr};
   for (int k = 0; k < tr->nstate; k++) uu[k] = (T *)u[k];
   for (int s = 0; s < nsteps; s++) {
-    for (int k = 0; k < tr->nstate; k++)
-      cudaMemcpyAsync(S.uold[k], uu[k], sizeof(T) * S.n, cudaMemcpyDeviceToDevice, S.st);
-    int rc = S.step(S.uold, uu, (T)dt);
+    int rc = S.step(uu, uu, (T)dt);
     if (rc) return gf_fail(ctx, rc, "RK step failed");
   }
   GF_CHECK_LAUNCH(ctx);
@@ -513,16 +476,16 @@ int advance(gf_problem *prob, const gf_rk_traits *tr, void *const *u, const void
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   GF_CUDA(ctx, cudaStreamIsCapturing(S.st, &cs));
   if (nsteps > 0 && cs == cudaStreamCaptureStatusNone) {
-    double *flag = prob->scal_d + RK_FLAG_SLOT;
-    GF_CUDA(ctx, cudaMemsetAsync(flag, 0, sizeof(double), S.st));
+    // the flag is in the problem's pinned host block: no memset, no copy back
+    volatile double *flag = prob->scal_h + RK_FLAG_SLOT;
+    *flag = 0.0;
     prob->launches++;
     k_nonfinite<T><<<grid_for(S.n, 256, ctx->sm_count * 8), 256, 0, S.st>>>(
-        S.n, tr->nstate, uu[0], uu[tr->nstate > 1 ? 1 : 0], uu[tr->nstate > 2 ? 2 : 0], flag);
+        S.n, tr->nstate, uu[0], uu[tr->nstate > 1 ? 1 : 0], uu[tr->nstate > 2 ? 2 : 0],
+        prob->scal_h + RK_FLAG_SLOT);
     GF_CHECK_LAUNCH(ctx);
-    GF_CUDA(ctx, cudaMemcpyAsync(prob->scal_h + RK_FLAG_SLOT, flag, sizeof(double),
-                                 cudaMemcpyDeviceToHost, S.st));
     GF_CUDA(ctx, cudaStreamSynchronize(S.st));
-    if (prob->scal_h[RK_FLAG_SLOT] != 0.0)
+    if (*flag != 0.0)
       return gf_fail(ctx, GF_ERR_NONFINITE, "solution not finite after %d RK steps", nsteps);
   }
   return GF_OK;

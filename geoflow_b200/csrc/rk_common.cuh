@@ -21,7 +21,7 @@ struct Stepper {
   int eqn, nstate, scheme;
   T nu;
   const T *c[3] = {nullptr, nullptr, nullptr};
-  T *uold[3] = {nullptr, nullptr, nullptr};
+  T *uacc[3] = {nullptr, nullptr, nullptr};
   T *utmp[3] = {nullptr, nullptr, nullptr};
   T *K[3][3] = {{nullptr}};
   // advection fast path (prescribed velocity, nu = 0, 2-d deformed or
@@ -46,21 +46,20 @@ struct Stepper {
   // false when the problem takes the separate RHS and update passes
   bool rhs_euler_smooth(T *const *u, T *const *x, T dt, T *const *uin, T a, T *const *y, T b,
                         T a2, T *const *y2, T b2, int *rc);
-  void smooth(T *v);
   // GMTK::constrain2sphere on the state where step_b calls it, on embedded
   // surfaces with node coordinates and a state of >= 3 components
+  bool constrains() const;
   void constrain(T *const *u);
-  // Smooth fused with the stage update before or after it
-  void euler_smooth(T *x, T dt, const T *uin, T a, const T *y, T b, T a2, const T *y2, T b2);
-  void smooth_accum(T *K, T ch, T *uout);
-  void accum_smooth(T *uout, const T *K, T ch);
-  // the same on every state component (arrays of nstate pointers; y and y2
-  // may be null): one pass over the lattice on box problems
+  // Smooth on every state component, in place or into out
   void smooth_n(T *const *v);
-  void euler_smooth_n(T *const *x, T dt, T *const *uin, T a, T *const *y, T b, T a2,
-                      T *const *y2, T b2);
-  void smooth_accum_n(T *const *K, T ch, T *const *uout);
-  void accum_smooth_n(T *const *uout, T *const *K, T ch);
+  void smooth_to(T *const *v, T *const *out);
+  // out = Smooth(the SSP substep update of x = dudt) (y and y2 may be null)
+  void euler_smooth_n(T *const *x, T *const *out, T dt, T *const *uin, T a, T *const *y, T b,
+                      T a2, T *const *y2, T b2);
+  // the class pass after a step_b stage (k_dss.cuh RK_MID, RK_MIDS, RK_LAST):
+  // K = Smooth(x), accout = accin + ch K, out = uin + b K or the step's result
+  void stage_pass(int mode, T *const *x, T *const *accin, T ch, T *const *accout, T *const *uin,
+                  T b, T *const *out);
   // One step uin -> uout.  With a tape (pointers tape[3*m + k], m = 0 ..
   // stages-1), stage m's input state (the argument of its RHS call) is left
   // in tape[3*m + k] for the adjoint sweep.

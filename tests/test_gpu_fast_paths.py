@@ -196,6 +196,55 @@ def test_line_applies(ctx, p, dim, geom):
             assert rel(out, ref) < tol, (vec, dt, rel(out, ref))
 
 
+@pytest.mark.parametrize("scheme", [A.GF_RK1, A.GF_RK2, A.GF_RK3, A.GF_RK4])
+def test_reverse_passes_box_equal_csr(ctx, scheme):
+    """The fused reverse class passes on a box against the CSR member lists."""
+    import torch
+    from geoflow_b200 import GBurgers, GridBox, Problem
+    g = GridBox(3, [3, 2, 4], 3, periodic=[1, 0, 1])
+    rng = np.random.default_rng(scheme)
+    u0 = [0.3 * rng.standard_normal(g.ndof()) for _ in range(3)]
+    obs = [0.3 * rng.standard_normal(g.ndof()) for _ in range(3)]
+    out = []
+    for s in (True, False):
+        prob = Problem(ctx, g, dirichlet_mask=False, structured=s)
+        B = GBurgers(prob, GBurgers.BURGERS, 1e-2, scheme=scheme)
+        out.append(B.adjoint_gradient([cuda(a, torch.float64) for a in u0], None,
+                                      [cuda(a, torch.float64) for a in obs], 1e-3, 5, 2))
+    (ja, ga), (jb, gb) = out
+    assert abs(ja - jb) <= 1e-13 * abs(jb)
+    for a, b in zip(ga, gb):
+        assert rel(a, b) < 1e-13
+
+
+@pytest.mark.parametrize("ne,p,per", [([33, 31, 33], 2, [0, 1, 0]), ([14, 11, 10], 6, [1, 0, 0]),
+                                      ([7, 8, 9], 9, [1, 1, 0]), ([75, 77], 7, [0, 0]),
+                                      ([262, 260], 2, [1, 0])])
+def test_lattice_runs_equal_csr(ctx, ne, p, per):
+    """Lattices of more than 2^18 points are walked in runs (smaller ones, point by
+    point): gathers and RK steps bit for bit as the member lists have them."""
+    import torch
+    from geoflow_b200 import GBurgers, GGFX, GridBox, Problem
+    g = GridBox(len(ne), ne, p, periodic=per)
+    rng = np.random.default_rng(p)
+    probs = [Problem(ctx, g, dirichlet_mask=False, structured=s) for s in (True, False)]
+    v = rng.standard_normal(g.ndof())
+    u0 = [0.3 * rng.standard_normal(g.ndof()) for _ in ne]
+    for dt in (torch.float64, torch.float32):
+        for op in (A.GF_DSS_SUM, A.GF_DSS_SMOOTH, A.GF_DSS_MAX, A.GF_DSS_MIN):
+            a, b = cuda(v, dt), cuda(v, dt)
+            assert GGFX(probs[0]).doOp(a, op) and GGFX(probs[1]).doOp(b, op)
+            assert bits_equal(a, b), (dt, op)
+        for scheme in (A.GF_RK2, A.GF_RK4, A.GF_SSP33):
+            us = []
+            for prob in probs:
+                u = [cuda(a, dt) for a in u0]
+                GBurgers(prob, A.GF_EQN_BURGERS, 1e-2, scheme=scheme).step(u, None, dt=1e-4, nsteps=1)
+                us.append(u)
+            for a, b in zip(*us):
+                assert bits_equal(a, b), (dt, scheme)
+
+
 @pytest.mark.parametrize("ne,p", [([33, 31, 33], 2), ([11, 10, 9], 7)])
 def test_multigrid_runs(ctx, ne, p):
     """Multigrid on more than 2^18 points against the Jacobi solve of the same grid
