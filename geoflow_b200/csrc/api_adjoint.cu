@@ -248,11 +248,134 @@ __global__ void __launch_bounds__(N *N *EPB)
   }
 }
 
+// The same on affine elements with D and K1 in even-odd form (k_dudt_aff.cuh):
+// along a line, with mu = Minv lam and c_d the direction's velocity,
+//   nu Jac X^2 W W (K1 mu) + Jac X W W D^T (W c_d mu)
+// and, for component m on direction m in Burgers, Jac X W W W sum_k (D u_k) mu_k:
+// half the multiply-adds of two full contractions (FP64 pipe), no per-node
+// geometry.  x- and y-lines go through shared memory to the z-column's owner.
+template <int N>
+struct VjpBasis {
+  AntiBasis<double, N> D, DT;
+  K1Basis<double, N> K;
+};
+template <int N, int EPB, int EQN>
+__global__ void __launch_bounds__(N *N *EPB)
+    k_dudt_vjp3a(const __grid_constant__ VjpBasis<N> B, const double *__restrict__ egeom,
+                 int64_t ne, double nu, const double *__restrict__ c0,
+                 const double *__restrict__ c1, const double *__restrict__ c2,
+                 const double *__restrict__ l0, const double *__restrict__ l1,
+                 const double *__restrict__ l2, const double *__restrict__ imass,
+                 double *__restrict__ o0, double *__restrict__ o1, double *__restrict__ o2) {
+  constexpr int NC = EQN == GF_EQN_BURGERS ? 3 : 1, NV = EQN == GF_EQN_HEAT ? 0 : 3;
+  constexpr int P = Pad<N>::P, PLANE = N * P, VOL = N * PLANE, NN = N * N, NNN = NN * N;
+  extern __shared__ __align__(16) double smv[];
+  double *sc = smv + threadIdx.y * (NV + NC + 2) * VOL;
+  double *smu = sc + NV * VOL, *sx = smu + NC * VOL, *sy = sx + VOL;
+  const int t = threadIdx.x, a0 = t % N, a1 = t / N;
+  const int64_t e = (int64_t)blockIdx.x * EPB + threadIdx.y;
+  const bool active = e < ne;
+  const int64_t base = e * NNN;
+  const int xl = a1 * PLANE + a0 * P, yl = a1 * PLANE + a0, zl = a1 * P + a0;
+  const double *cin[3] = {c0, c1, c2}, *lin[3] = {l0, l1, l2};
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const int64_t node = base + k * NN + t;
+    const double im = active ? imass[node] : 0.0;
+#pragma unroll
+    for (int v = 0; v < NV; v++) sc[v * VOL + zl + k * PLANE] = active ? cin[v][node] : 0.0;
+#pragma unroll
+    for (int m = 0; m < NC; m++) smu[m * VOL + zl + k * PLANE] = active ? im * lin[m][node] : 0.0;
+  }
+  double X[3] = {0.0, 0.0, 0.0}, J = 0.0;
+  if (active) {
+    const double *ge = egeom + e * 4;
+    X[0] = ge[0];
+    X[1] = ge[1];
+    X[2] = ge[2];
+    J = ge[3];
+  }
+  const double w2 = J * (B.K.W[a0] * B.K.W[a1]);
+  __syncthreads();
+  const int s0[3] = {xl, yl, zl}, st[3] = {1, P, PLANE};
+  const double ca[3] = {w2 * X[0], w2 * X[1], w2 * X[2]};
+  const double cd[3] = {nu * (ca[0] * X[0]), nu * (ca[1] * X[1]), nu * (ca[2] * X[2])};
+#pragma unroll
+  for (int m = 0; m < NC; m++) {
+    // the x-, y- and z-lines of component m together (lines_K1)
+    double r[3][N], mid[3];
+    double2 eo[3][N / 2];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      double a[N];
+#pragma unroll
+      for (int q = 0; q < N; q++) a[q] = smu[m * VOL + s0[d] + q * st[d]];
+      line_eo<double, N>(a, eo[d]);
+      mid[d] = a[(N - 1) / 2];
+    }
+    lines_K1<double, N, 3>(B.K, eo, mid, cd, [&](int l, int i, double v) { r[l][i] = v; });
+    if (NV) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        double a[N];
+#pragma unroll
+        for (int q = 0; q < N; q++)
+          a[q] = B.K.W[q] * sc[d * VOL + s0[d] + q * st[d]] * smu[m * VOL + s0[d] + q * st[d]];
+        line_eo<double, N>(a, eo[d]);
+        mid[d] = a[(N - 1) / 2];
+      }
+      lines_anti<double, N, 3>(B.DT, eo, mid, [&](int l, int i, double v) {
+        r[l][i] = fma(ca[l], v, r[l][i]);
+      });
+    }
+    if (EQN == GF_EQN_BURGERS) {  // sum_k (D_m u_k) mu_k on the lines of direction m
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        double a[N];
+#pragma unroll
+        for (int q = 0; q < N; q++) a[q] = sc[k * VOL + s0[m] + q * st[m]];
+        line_eo<double, N>(a, eo[k]);
+        mid[k] = a[(N - 1) / 2];
+      }
+      lines_anti<double, N, 3>(B.D, eo, mid, [&](int k, int i, double v) {
+        r[m][i] = fma(ca[m] * B.K.W[i] * smu[k * VOL + s0[m] + i * st[m]], v, r[m][i]);
+      });
+    }
+#pragma unroll
+    for (int q = 0; q < N; q++) {
+      sx[xl + q] = r[0][q];
+      sy[yl + q * P] = r[1][q];
+    }
+    __syncthreads();
+    if (active) {
+      double *o = m == 0 ? o0 : (m == 1 ? o1 : o2);
+#pragma unroll
+      for (int k = 0; k < N; k++)
+        o[base + k * NN + t] = -((sx[zl + k * PLANE] + sy[zl + k * PLANE]) + r[2][k]);
+    }
+    if (m + 1 < NC) __syncthreads();
+  }
+}
+
 template <int N, int DIM, int EQN>
 int launch_vjp_n(gf_problem *prob, double nu, const double *const *c, const double *const *lam,
                  double *const *out, cudaStream_t st) {
   const Basis<double, N> B = make_basis<double, N>(prob);
   const Geom<double> g = geom_of<double>(prob);
+  if (DIM == 3 && g.egeom && prob->d_antisym) {
+    constexpr int EPB = epb_aff<double, N>();
+    constexpr int NF = (EQN == GF_EQN_HEAT ? 0 : 3) + (EQN == GF_EQN_BURGERS ? 3 : 1) + 2;
+    const size_t smem = sizeof(double) * NF * N * N * Pad<N>::P * EPB;
+    const VjpBasis<N> VB{make_antibasis<double, N>(prob, false),
+                         make_antibasis<double, N>(prob, true), make_k1basis<double, N>(prob)};
+    auto kern = k_dudt_vjp3a<N, EPB, EQN>;
+    set_smem(kern, smem);
+    prob->launches++;
+    kern<<<(unsigned)((prob->ne + EPB - 1) / EPB), dim3(N * N, EPB), smem, st>>>(
+        VB, g.egeom, prob->ne, nu, c[0], c[1], c[2], lam[0], lam[1], lam[2], prob->imass_d, out[0],
+        out[1], out[2]);
+    return cudaPeekAtLastError() == cudaSuccess ? GF_OK : GF_ERR_CUDA;
+  }
   if (DIM == 3) {
     constexpr int EPB = epb_vjp3<N>();
     constexpr int NF = (EQN == GF_EQN_HEAT ? 0 : 3) + (EQN == GF_EQN_BURGERS ? 3 : 1) + 2;
