@@ -18,6 +18,7 @@
 #include "k_dss.cuh"
 #include "k_vec.cuh"
 #include "ops_launch.cuh"
+#include "rk_cluster.cuh"
 #include "rk_common.cuh"
 #include "rk_pass.cuh"
 
@@ -430,6 +431,74 @@ int Stepper<T>::step_ssp(T *const *uin, T *const *uout, T dt) {
   return GF_OK;
 }
 
+// Small 2-d boxes with a diagonal metric take all steps in one cluster
+// (rk_cluster.cuh); step_b of order 1 smooths its input first and does not.
+template <typename T>
+bool Stepper<T>::cluster_ok() const {
+  BoxWalk w;
+  return prob->dim == 2 && prob->geom <= GF_GEOM_REGULAR && scheme != GF_RK1 &&
+         n * nstate <= RKC_NODES && dss_box_walk(prob, w);
+}
+
+template <typename T>
+int Stepper<T>::cluster_steps(T *const *u, T dt, int nsteps) {
+  RKProgram<T> pr{};
+  pr.nsteps = nsteps;
+  pr.nc = nstate;
+  pr.c[0] = c[0];
+  pr.c[1] = c[1];
+  pr.imass = imass_of<T>(prob);
+  pr.g = geom_of<T>(prob);
+  pr.ne = prob->ne;
+  pr.nu = nu;
+  pr.nph = stages();
+  auto set = [&](auto &dst, T *const *src) {
+    for (int k = 0; k < nstate; k++) dst[k] = src[k];
+  };
+  if (scheme <= 4) {  // step()'s stages, in place
+    double alpha[4], beta[4][4], cc[4];
+    butcher(scheme, alpha, beta, cc);
+    for (int m = 0; m < scheme; m++) {
+      RKPhase<T> &h = pr.ph[m];
+      set(h.in, m ? (T *const *)utmp : u);
+      set(h.out, K[0]);
+      set(h.pass.x, K[0]);
+      set(h.pass.accin, m ? (T *const *)uacc : u);
+      h.pass.ch = (T)cc[m] * dt;
+      if (m == scheme - 1) {
+        h.mode = RK_LAST;
+        set(h.pass.out, u);
+        continue;
+      }
+      h.mode = m == scheme - 2 ? RK_MIDS : RK_MID;
+      set(h.pass.acc, uacc);
+      set(h.pass.uin, u);
+      set(h.pass.out, utmp);
+      h.pass.b = (T)beta[m + 1][m] * dt;
+    }
+  } else {
+    for (int m = 0; m < pr.nph; m++) {
+      RKPhase<T> &h = pr.ph[m];
+      const SSPSubstep<T> q = ssp_coeffs<T>(scheme, m);
+      auto state = [&](int i) { return i == 0 ? u : (T *const *)K[i - 1]; };  // stage inputs
+      set(h.in, state(m));
+      set(h.out, utmp);
+      h.mode = RK_EULER;
+      set(h.pass.x, utmp);
+      set(h.pass.uin, state(m));
+      if (q.y >= 0) set(h.pass.y, state(q.y));
+      if (q.y2 >= 0) set(h.pass.y2, state(q.y2));
+      set(h.pass.out, m + 1 < pr.nph ? (T *const *)K[m] : u);
+      h.pass.dt = dt;
+      h.pass.a = q.a;
+      h.pass.b = q.b;
+      h.pass.a2 = T(1);
+      h.pass.b2 = q.b2;
+    }
+  }
+  return launch_rk_cluster<T>(prob, eqn, pr, st);
+}
+
 template struct Stepper<double>;
 template struct Stepper<float>;
 
@@ -463,9 +532,14 @@ int advance(gf_problem *prob, const gf_rk_traits *tr, void *const *u, const void
   S.prepare_adv();  // advection with a prescribed velocity and nu = 0
   T *uu[3] = {nullptr, nullptr, nullptr};
   for (int k = 0; k < tr->nstate; k++) uu[k] = (T *)u[k];
-  for (int s = 0; s < nsteps; s++) {
-    int rc = S.step(uu, uu, (T)dt);
-    if (rc) return gf_fail(ctx, rc, "RK step failed");
+  if (nsteps > 0 && S.cluster_ok()) {
+    int rc = S.cluster_steps(uu, (T)dt, nsteps);
+    if (rc) return gf_fail(ctx, rc, "RK steps failed");
+  } else {
+    for (int s = 0; s < nsteps; s++) {
+      int rc = S.step(uu, uu, (T)dt);
+      if (rc) return gf_fail(ctx, rc, "RK step failed");
+    }
   }
   GF_CHECK_LAUNCH(ctx);
   // The reference asserts a finite state after every step; a NaN or Inf

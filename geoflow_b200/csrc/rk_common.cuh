@@ -65,6 +65,9 @@ struct Stepper {
   // in tape[3*m + k] for the adjoint sweep.
   int step(T *const *uin, T *const *uout, T dt, T *const *tape = nullptr);
   int step_ssp(T *const *uin, T *const *uout, T dt);
+  // nsteps steps in place in one launch, where cluster_ok()
+  bool cluster_ok() const;
+  int cluster_steps(T *const *u, T dt, int nsteps);
   int stages() const { return scheme <= 4 ? scheme : (scheme == GF_SSP22 ? 2 : (scheme == GF_SSP33 ? 3 : 4)); }
 };
 

@@ -91,6 +91,30 @@ def test_rhs_with_an_asymmetric_derivative_matrix(ctx):
         assert rel(a, b) < 1e-12
 
 
+@pytest.mark.parametrize("ne,p,per", [([1, 3], 1, [0, 1]), ([16, 16], 4, [1, 1]), ([5, 3], 11, [0, 0]),
+                                      ([17, 9], 6, [1, 0]), ([2, 40], 2, [0, 1]), ([3, 2], 9, [1, 1])])
+@pytest.mark.parametrize("scheme", [A.GF_RK2, A.GF_RK3, A.GF_RK4, A.GF_SSP22, A.GF_SSP33, A.GF_SSP34])
+def test_cluster_steps_equal_separate_kernels(ctx, ne, p, per, scheme):
+    import torch
+    from geoflow_b200 import GBurgers, GridBox, Problem
+    g = GridBox(2, ne, p, periodic=per)
+    rng = np.random.default_rng(p + scheme)
+    for geom in ("affine", "regular"):
+        probs = [Problem(ctx, g, structured=s, geometry=geom) for s in (True, False)]
+        for eqn, ns in ((A.GF_EQN_ADVECT, 1), (A.GF_EQN_BURGERS, 2), (A.GF_EQN_HEAT, 1)):
+            u0 = [0.3 * rng.standard_normal(g.ndof()) for _ in range(ns)]
+            c0 = [rng.standard_normal(g.ndof()) for _ in range(2)]
+            for dt in (torch.float64, torch.float32):
+                c = [cuda(a, dt) for a in c0] if eqn == A.GF_EQN_ADVECT else None
+                us = []
+                for prob in probs:
+                    u = [cuda(a, dt) for a in u0]
+                    GBurgers(prob, eqn, 1e-2, scheme=scheme).step(u, c, dt=1e-4, nsteps=3)
+                    us.append(u)
+                for a, b in zip(*us):
+                    assert bits_equal(a, b), (geom, eqn, dt)
+
+
 @pytest.mark.parametrize("ne,p,per", [([2, 3], 1, [0, 0]), ([8, 8], 3, [0, 0]), ([32, 32], 5, [0, 0]),
                                       ([5, 7], 11, [1, 0]), ([1, 4], 6, [1, 0]), ([40, 3], 2, [0, 1]),
                                       ([9, 6], 8, [0, 0])])
