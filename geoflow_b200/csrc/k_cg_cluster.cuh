@@ -124,8 +124,9 @@ __host__ __device__ inline size_t cl_slab_bytes(int M0, int M1, int P, int ctas)
 }
 constexpr size_t CL_SLAB_MAX = 208 * 1024;
 // Lattice points up to which one cluster beats the whole chip with a launch per
-// pass: a solve on 60 k points, p = 7, takes 2.40 ms against 2.84, on 79 k,
-// p = 4, 1.34 against 1.61, on 99 k, p = 7, 4.88 against 4.40.
+// pass (as measured with the passes of that time, 10 % slower than now): a solve
+// on 60 k points, p = 7, takes 2.38 ms against 2.84, on 79 k, p = 4, 1.35 against
+// 1.61; on 99 k, p = 7, 4.88 against 3.85 with the passes of now.
 constexpr int64_t CL_NODES = 80000;
 
 inline ClProblem cl_problem(const BoxLattice &L) {
