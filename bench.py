@@ -404,7 +404,7 @@ def e2e_solve(ctx, prob, H, b, traits, reps=2):
 # ---------------------------------------------------------------------------
 def rk_stage_bench(ctx, ne, p, steps=3, warmup=2):
     """SSP-RK3 Burgers on a periodic box: GDOF/s per stage in FP32 and FP64,
-    the stage split into its two kernels (the fused RHS k_dudt3d, timed
+    the stage split into its two kernels (the fused RHS k_dudt3a, timed
     alone through gf_dudt, and the rest of the stage: the stage update and
     Smooth pass; in FP32 the stage's RHS kernel carries the update as its
     epilogue, so there the RHS-alone figure is the kernel without it) with
@@ -459,14 +459,14 @@ def rk_stage_bench(ctx, ne, p, steps=3, warmup=2):
         del K
         out[name] = {"ms_per_stage": t_stage * 1e3,
                      "gdofs_per_stage": 3 * n / t_stage / 1e9,
-                     "stage_kernels": ("k_dudt3d with the SSP update epilogue, then the "
-                                       "Smooth k_dss_smooth_box_n" if name == "f32" else
-                                       "k_dudt3d, then the stage update and Smooth "
-                                       "k_dss_rk_box_n"),
+                     "stage_kernels": ("k_dudt3a with the SSP update epilogue, then the "
+                                       "Smooth pass k_rk_box" if name == "f32" else
+                                       "k_dudt3a, then the stage update and Smooth "
+                                       "pass k_rk_box"),
                      "kernels": {
-                         "k_dudt3d": {"ms": t_rhs * 1e3, "alg_bytes": rhs_bytes,
+                         "k_dudt3a": {"ms": t_rhs * 1e3, "alg_bytes": rhs_bytes,
                                       "gbs": rhs_bytes / t_rhs / 1e9},
-                         "k_dss_rk_box_n (stage - rhs)": {"ms": t_upd * 1e3,
+                         "k_rk_box (stage - rhs)": {"ms": t_upd * 1e3,
                                                           "alg_bytes": upd_bytes,
                                                           "gbs": upd_bytes / t_upd / 1e9}}}
         del uu

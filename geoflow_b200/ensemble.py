@@ -4,8 +4,8 @@ The reference runs one problem per process; an ensemble runs many small
 ones at once on one GPU: one persistent cooperative launch per RK stage of
 every member (deformed / embedded 2-d members, e.g. icosahedral-sphere
 advection) or per CG iteration of every member (2-d box Helmholtz solves:
-FP64 iterations, or FP32 iterations with FP64 residual refinement),
-captured in CUDA graphs.
+FP32 iterations with FP64 residual refinement, or FP64 iterations), captured
+in CUDA graphs.  Small members with FP64 iterations take one launch per solve.
 """
 from __future__ import annotations
 

@@ -505,7 +505,8 @@ int gf_adjoint_gradient(gf_problem_t prob, const gf_rk_traits *traits,
 /* ---- ensembles of independent problems (no reference counterpart: the
  * reference runs one problem per process) ----
  * Up to 64 2-d members of orders 2..9 advanced together, one persistent
- * cooperative launch per RK stage or CG iteration, captured in CUDA graphs.
+ * cooperative launch per RK stage or CG iteration, captured in CUDA graphs
+ * (small members with FP64 iterations: one launch per solve, a cluster each).
  * Members are either all deformed / embedded problems (GF_ENS_RK: e.g.
  * icosahedral-sphere advection, each member bit-identical to gf_rk_advance
  * on it alone) or all box problems with affine elements (GF_ENS_CG:
