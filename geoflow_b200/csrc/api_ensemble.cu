@@ -26,7 +26,7 @@
 // and do not depend on the launch shape.
 //
 // Arithmetic.  An RK member's element body is def_element (k_def.cuh), its
-// folds are those of k_dss_rk_split / k_dss_split and its stage sums those of
+// folds are those of k_rk_split / k_dss_split and its stage sums those of
 // step_b (rk_stage_point), so each member advances bit for bit as
 // gf_rk_advance advances it alone.  A CG member runs GCG::solve_impl's DFM
 // iteration (solvers/gcg.ipp:239-382) with a Jacobi preconditioner on the
@@ -271,7 +271,7 @@ struct LoadFinal {
 // member is finished here (its fold is (0 + v) / 1: K = that, and uout +=
 // c h K, or in the last stage uout = Smooth(uout + c h K)); a node of a
 // shared class keeps the raw slope for the fold after the barrier.  The
-// arithmetic is that of k_dss_rk_split, node for node.
+// arithmetic is that of k_rk_split, node for node.
 template <typename T>
 struct OutStage {
   const float *imult;
@@ -382,7 +382,7 @@ __device__ void en_rk_elements(const EnArgs &a, const int64_t *cpref, bool from_
 // several members (shared nodes; a class of one member is finished by the
 // element phase), one thread each from the problem's shared-class list
 // (sh_ptr / sh_members, members in ascending local id), numbered over all
-// members (prefix spref).  The fold is that of k_dss_rk_split: from 0, in
+// members (prefix spref).  The fold is that of k_rk_split: from 0, in
 // member order, divided by the count.
 template <class FC>
 __device__ __forceinline__ void en_rk_items(const EnArgs &a, const int64_t *spref, FC cls) {
