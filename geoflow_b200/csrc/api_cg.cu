@@ -1175,8 +1175,8 @@ enum { DP_NONE = 0, DP_X = 1, DP_D = 2 };
 // copies of a point are added in the (z, y, x) nesting (ascending element id
 // unless a periodic direction has a single element).  One thread per point
 // executed 133 instructions per point, most of them index arithmetic.
-// (ONE: a point per thread, RunWalk::one; in one kernel with the runs it cost them
-// registers, FP32 p = 7 step 60 -> 80 us.)
+// ONE: a point per thread, RunWalk::one.  One loop for either walk: with the body
+// as a lambda of two loops the FP32 p = 7 step took 80 us in place of 60.
 template <int N, int MODE, bool DOTS, typename TM, bool ONE>
 __global__ void __launch_bounds__(RED_THREADS)
     k_mg_pass_lat(const RunWalk<N - 1> w, Weights wt,
@@ -1188,7 +1188,10 @@ __global__ void __launch_bounds__(RED_THREADS)
   if (scal[S_DONE] != 0.0) return;
   constexpr int P = N - 1;
   double rz = 0.0;
-  auto pass = [&](const LatRun &k) {
+  const int nt = ONE ? w.npts : w.n, stride = gridDim.x * blockDim.x;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nt;
+       t = (t < nt - stride) ? t + stride : nt) {
+    const LatRun k = ONE ? w.point(t) : w.run(t);
     TM s[P] = {}, bc[P] = {}, dv[P] = {}, xo[P] = {}, dp[P] = {};
     bool keep[P];
 #pragma unroll
@@ -1227,12 +1230,6 @@ __global__ void __launch_bounds__(RED_THREADS)
         if (DOTS) rz += (double)bc[r] * (double)xc;
       }
     }
-  };
-  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-  if (ONE) {
-    for (int t = t0; t < w.npts; t = (t < w.npts - stride) ? t + stride : w.npts) pass(w.point(t));
-  } else {
-    for (int t = t0; t < w.n; t = (t < w.n - stride) ? t + stride : w.n) pass(w.run(t));
   }
   if (!DOTS) return;
   rz = block_reduce<false>(rz, sh);
