@@ -1533,9 +1533,11 @@ struct Solver {
     });
   }
 
-  // small 2-d affine boxes iterate inside one cluster (CL_NODES)
+  // small 2-d affine boxes iterate inside one cluster (CL_NODES), whose lines take
+  // K1, the operator of a centro-antisymmetric D alone
   bool cluster_ok() {
-    if (MAP::NPTS == 0 || prob->dim != 2 || !prob->egeom_d || nL > CL_NODES) return false;
+    if (MAP::NPTS == 0 || prob->dim != 2 || !prob->egeom_d || !prob->d_antisym || nL > CL_NODES)
+      return false;
     if constexpr (MAP::NPTS > 0)
       if (ctx->cluster_size == 0)
         ctx->cluster_size = cl_cluster_size(k_cg_cluster<MAP::NPTS>, CL_THREADS);

@@ -1916,18 +1916,22 @@ extern "C" int gf_ensemble_cg_solve(gf_ensemble_t E, const gf_cg_traits *tr, dou
     E->launches++;
   }
   // FP64 members whose direction fits the shared memory of a cluster (about 250 k
-  // points): a cluster per member and one launch for the whole solve.  Twelve
+  // points) and whose D is centro-antisymmetric (the cluster's lines take K1, which
+  // is the operator of no other D): a cluster per member and one launch for the whole
+  // solve.  Twelve
   // members, the largest of 201 k points: 7.0 ms against 9.4 with the grid-wide
   // iteration, which costs 65-75 us whatever the members.
   size_t slab = 0;
-  if (a.fp64) {
+  const bool cluster = a.fp64 && std::all_of(E->probs.begin(), E->probs.end(),
+                                             [](const gf_problem *m) { return m->d_antisym; });
+  if (cluster) {
     if (ctx->cluster_size == 0) ctx->cluster_size = cl_cluster_size(k_en_cg_cluster, CL_THREADS);
     for (int m = 0; m < n; m++) {
       const EnMember &M = E->host[m];
       slab = std::max(slab, cl_slab_bytes(M.walk.M[0], M.walk.M[1], M.N - 1, ctx->cluster_size));
     }
   }
-  if (a.fp64 && slab <= CL_SLAB_MAX) {
+  if (cluster && slab <= CL_SLAB_MAX) {
     GF_CUDA(ctx, cudaFuncSetAttribute(k_en_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)slab));
     if (ctx->cluster_size == CL_MAX)

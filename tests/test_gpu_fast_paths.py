@@ -148,6 +148,52 @@ def test_cluster_cg_equals_separate_kernels(ctx, ne, p, per, norm):
             assert abs(ha[0] - hb[0]) <= 1e-9 * hb[0]
 
 
+def asymmetric_grid(ne, p, **kw):
+    """A box whose derivative matrix is not centro-antisymmetric."""
+    from geoflow_b200 import GridBox
+    g = GridBox(len(ne), ne, p, **kw)
+    g.D = g.D * (1.0 + 0.1 * np.random.default_rng(p).standard_normal(g.D.size))
+    return g
+
+
+@pytest.mark.parametrize("ne,p", [([2, 3], 2), ([6, 5], 4), ([4, 4], 7)])
+def test_solves_with_an_asymmetric_derivative_matrix(ctx, ne, p):
+    """The 2-d FP64 solves, alone and in an ensemble, solve with the operator of
+    opVec_prod: as the same grid without its box description, and the assembled
+    residual by opVec_prod vanishes."""
+    import torch
+    from geoflow_b200 import CGTraits, Ensemble, GCG, GGFX, GHelmholtz, Problem
+    g = asymmetric_grid(ne, p)
+    probs = [Problem(ctx, g, structured=s) for s in (True, False)]
+    b = cuda(np.random.default_rng(p).standard_normal(g.ndof()), torch.float64)
+    tr = CGTraits(maxit=4000, normtype=A.GF_NORM_EUC, tol=1e-11, relative=1,
+                  precond=A.GF_PRECOND_JACOBI, precision=A.GF_CG_FP64)
+    xs = []
+    for prob in probs:
+        H = GHelmholtz(prob)
+        H.set_Lap_scalar(0.3)
+        H.set_mass_scalar(2.0)
+        x = prob.zeros()
+        assert GCG(tr, prob).solve(H, b, prob.zeros(), x) == 0
+        xs.append(x)
+    xe = probs[0].zeros()
+    rc, _, _, st = Ensemble(ctx, probs[:1]).solve([b], [xe], tr, p=0.3, q=2.0)
+    assert rc == 0 and list(st) == [0]
+    assert rel(xs[0], xs[1]) < 1e-8
+    assert rel(xe, xs[1]) < 1e-8
+    H = GHelmholtz(probs[1])
+    H.set_Lap_scalar(0.3)
+    H.set_mass_scalar(2.0)
+    for x in (xs[0], xe):
+        ax = probs[1].zeros()
+        H.opVec_prod(x, None, ax)
+        r = (b - ax) * cuda(g.mask, torch.float64)
+        s = b.clone()
+        for v in (r, s):
+            GGFX(probs[1]).doOp(v, GGFX.Sum)
+        assert float((r * cuda(g.mask, torch.float64)).abs().max()) < 1e-9 * float(s.abs().max())
+
+
 def test_cluster_cg_outcomes(ctx):
     """maxit, an exact start and a non-finite right-hand side."""
     import torch
