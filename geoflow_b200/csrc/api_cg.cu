@@ -2042,6 +2042,7 @@ int mg_light_problem(gf_context *ctx, int dim, const int (&ne)[3], const int (&p
   std::vector<double> xi(n);
   gf_gll_basis(p, xi.data(), lp->W, lp->D);
   gfk::gf_k1_matrix(n, lp->D, lp->W, lp->K1);
+  lp->d_antisym = true;  // a GLL basis
   BoxLattice L{};
   L.dim = dim;
   L.p = p;

@@ -91,7 +91,8 @@ struct HelmLaunch {
       const Geom<T> g = geom_of<T>(prob);
       constexpr int P = Pad<N>::P;
       if constexpr (std::is_same<T, float>::value && N == 8) {
-        if (prob->dim == 3 && g.egeom && !pvec && g_fp32_apply_mode == GF_FP32_APPLY_TF32) {
+        if (prob->dim == 3 && g.egeom && !pvec && prob->d_antisym &&
+            g_fp32_apply_mode == GF_FP32_APPLY_TF32) {
           // affine elements, scalar p, p = 7: the K1 contractions as 3xTF32
           // tensor-core products (k_helm_tf32.cuh)
           constexpr int EPB = 4;
@@ -103,8 +104,9 @@ struct HelmLaunch {
           return GF_OK;
         }
       }
-      if (prob->dim == 3 && g.egeom && !pvec) {
-        // affine elements, scalar p: one K1 contraction per direction
+      if (prob->dim == 3 && g.egeom && !pvec && prob->d_antisym) {
+        // affine elements, scalar p: one K1 contraction per direction, in the
+        // even-odd form that only a centro-antisymmetric D has
         constexpr int EPB = epb_k1<N>();
         const K1Basis<T, N> KB = make_k1basis<T, N>(prob);
         const size_t smem = sizeof(T) * 2 * N * N * P * EPB;

@@ -156,6 +156,49 @@ def asymmetric_grid(ne, p, **kw):
     return g
 
 
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("p", [1, 2, 5, 7, 8])
+def test_applies_with_an_asymmetric_derivative_matrix(ctx, dim, p):
+    """The affine apply, by FMA and (p = 7) by tensor cores, against the per-node
+    kernel of the same grid; then a solve with each preconditioner."""
+    import torch
+    from geoflow_b200 import CGTraits, GCG, GHelmholtz, Problem
+    g = asymmetric_grid([3, 2, 2][:dim], p, length=[1.0, 0.7, 1.3][:dim])
+    u = np.random.default_rng(p).standard_normal(g.ndof())
+    probs = [Problem(ctx, g, geometry=geom) for geom in ("affine", "regular")]
+    Hs = [GHelmholtz(prob) for prob in probs]
+    for H in Hs:
+        H.set_Lap_scalar(0.6)
+        H.set_mass_scalar(1.7)
+    lib = A.load()
+    for dt, mode, tol in ((torch.float64, A.GF_FP32_APPLY_FMA, 1e-12),
+                          (torch.float32, A.GF_FP32_APPLY_FMA, 2e-5),
+                          (torch.float32, A.GF_FP32_APPLY_TF32, 2e-5)):
+        prev = lib.gf_set_fp32_apply(mode)
+        try:
+            out = []
+            for prob, H in zip(probs, Hs):
+                o = prob.zeros(dt)
+                H.opVec_prod(cuda(u, dt), None, o)
+                out.append(o)
+        finally:
+            lib.gf_set_fp32_apply(prev)
+        assert rel(*out) < tol, (dt, mode, rel(*out))
+    b = cuda(np.random.default_rng(p + 1).standard_normal(g.ndof()), torch.float64)
+    kinds = [(1, A.GF_PRECOND_JACOBI, A.GF_CG_FP64), (0, A.GF_PRECOND_JACOBI, A.GF_CG_FP64)]
+    if dim == 3 and p >= 5:  # enough unknowns for a batch of FP32 iterations
+        kinds += [(0, A.GF_PRECOND_JACOBI, A.GF_CG_MIXED), (0, A.GF_PRECOND_PMG, A.GF_CG_FP64)]
+    xs = []
+    for i, pre, prec in kinds:
+        x = probs[i].zeros()
+        tr = CGTraits(maxit=8000, normtype=A.GF_NORM_EUC, tol=1e-11, relative=1, precond=pre,
+                      precision=prec)
+        assert GCG(tr, probs[i]).solve(Hs[i], b, probs[i].zeros(), x) == 0, (pre, prec)
+        xs.append(x)
+    for x in xs[1:]:
+        assert rel(x, xs[0]) < 1e-8
+
+
 @pytest.mark.parametrize("ne,p", [([2, 3], 2), ([6, 5], 4), ([4, 4], 7)])
 def test_solves_with_an_asymmetric_derivative_matrix(ctx, ne, p):
     """The 2-d FP64 solves, alone and in an ensemble, solve with the operator of
