@@ -517,7 +517,7 @@ struct Reverse {
   static int slots(int nstate) { return nstate * 7; }
   // Smooth (its own transpose) on every state component: one lattice pass
   // on box problems (the stepper's multi-component kernel), CSR otherwise
-  void smooth_n(double *const *v) { S.smooth_n(v); }
+  int smooth_n(double *const *v) { return S.smooth_n(v); }
 
   // lam <- (d step/d uin)^T lam; tape[3*m + k] = input of stage m
   int run(double *const *tape, double *const *lam, double dt) {
@@ -543,18 +543,20 @@ struct Reverse {
       p.out[k] = mu[k];
     }
     p.ch = cc[ns - 1] * h;
-    rk_pass<double>(prob, ADJ_START, nstate, p, st);
+    int rc = rk_pass<double>(prob, ADJ_START, nstate, p, st);
+    if (rc) return rc;
     for (int k = 0; k < nstate; k++) p.x[k] = tmp[k];
     for (int m = ns - 1; m >= 0; m--) {
       const double *um[3] = {tape[3 * m], tape[3 * m + 1], tape[3 * m + 2]};
-      int rc = vjp(prob, S.eqn, (double)S.nu, nstate, um, S.c, (const double *const *)mu, tmp);
+      rc = vjp(prob, S.eqn, (double)S.nu, nstate, um, S.c, (const double *const *)mu, tmp);
       if (rc) return rc;
       if (m == 0) break;
       p.ch = cc[m - 1] * h;
       p.b = beta[m][m - 1] * h;
-      rk_pass<double>(prob, m == ns - 1 ? ADJ_STAGE_LAST : ADJ_STAGE, nstate, p, st);
+      rc = rk_pass<double>(prob, m == ns - 1 ? ADJ_STAGE_LAST : ADJ_STAGE, nstate, p, st);
+      if (rc) return rc;
     }
-    if (ns == 1) smooth_n(tmp);
+    if (ns == 1 && (rc = smooth_n(tmp))) return rc;
     for (int k = 0; k < nstate; k++) p.out[k] = lam[k];
     prob->launches++;
     k_adj_add<<<g, 256, 0, st>>>(n, nstate, p);
@@ -591,9 +593,10 @@ struct Reverse {
         cudaMemsetAsync(lamK[m][k], 0, sizeof(double) * n, st);
     double *lout[3] = {lam[0], lam[1], lam[2]};  // cotangent of out_m
     for (int m = ns - 1; m >= 0; m--) {
-      smooth_n(lout);
+      int rc = smooth_n(lout);
+      if (rc) return rc;
       const double *um[3] = {tape[3 * m], tape[3 * m + 1], tape[3 * m + 2]};
-      int rc = vjp(prob, S.eqn, (double)S.nu, nstate, um, S.c, (const double *const *)lout, tmp);
+      rc = vjp(prob, S.eqn, (double)S.nu, nstate, um, S.c, (const double *const *)lout, tmp);
       if (rc) return rc;
       double a, b, b2;
       int y, y2;

@@ -1167,11 +1167,7 @@ const void *en_kernel(int which) {
 int en_grid(gf_ensemble *E, int which, int threads, int bps, int wbytes) {
   const void *k = en_kernel(which);
   const size_t smem = (size_t)wbytes * (threads / 32);
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
+  if (!set_smem_of(k, smem)) return 0;
   int occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, threads, smem) != cudaSuccess) {
     cudaGetLastError();
@@ -1182,11 +1178,7 @@ int en_grid(gf_ensemble *E, int which, int threads, int bps, int wbytes) {
   const void *other = which == 0   ? (const void *)k_en_rk_tune<double>
                       : which == 1 ? (const void *)k_en_rk_tune<float>
                                    : (const void *)k_en_cg_init;
-  if (cudaFuncSetAttribute(other, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
+  if (!set_smem_of(other, smem)) return 0;
   if (which == 2) {
     int occ2 = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, other, threads, smem) != cudaSuccess) {

@@ -239,30 +239,29 @@ bool Stepper<T>::rhs_euler_smooth(T *const *u, T *const *x, T dt, T *const *uin,
     const RKEpi<T> e = epi_for(0, nstate);
     if ((*rc = launch_dudt<T>(prob, eqn, MODE_EULER, nu, f, o, st, &e))) return true;
   }
-  smooth_to(utmp, x);
-  *rc = GF_OK;
+  *rc = smooth_to(utmp, x);
   return true;
 }
 
 // v <- Smooth(v) in place
 template <typename T>
-void Stepper<T>::smooth_n(T *const *v) {
-  smooth_to(v, v);
+int Stepper<T>::smooth_n(T *const *v) {
+  return smooth_to(v, v);
 }
 
 template <typename T>
-void Stepper<T>::smooth_to(T *const *v, T *const *out) {
+int Stepper<T>::smooth_to(T *const *v, T *const *out) {
   RKPass<T> p{};
   for (int k = 0; k < nstate; k++) {
     p.x[k] = v[k];
     p.out[k] = out[k];
   }
-  rk_pass<T>(prob, RK_SMOOTH, nstate, p, st);
+  return rk_pass<T>(prob, RK_SMOOTH, nstate, p, st);
 }
 
 template <typename T>
-void Stepper<T>::euler_smooth_n(T *const *x, T *const *out, T dt, T *const *uin, T a, T *const *y,
-                                T b, T a2, T *const *y2, T b2) {
+int Stepper<T>::euler_smooth_n(T *const *x, T *const *out, T dt, T *const *uin, T a, T *const *y,
+                               T b, T a2, T *const *y2, T b2) {
   RKPass<T> p{};
   for (int k = 0; k < nstate; k++) {
     p.x[k] = x[k];
@@ -276,12 +275,12 @@ void Stepper<T>::euler_smooth_n(T *const *x, T *const *out, T dt, T *const *uin,
   p.b = b;
   p.a2 = a2;
   p.b2 = b2;
-  rk_pass<T>(prob, RK_EULER, nstate, p, st);
+  return rk_pass<T>(prob, RK_EULER, nstate, p, st);
 }
 
 template <typename T>
-void Stepper<T>::stage_pass(int mode, T *const *x, T *const *accin, T ch, T *const *accout,
-                            T *const *uin, T b, T *const *out) {
+int Stepper<T>::stage_pass(int mode, T *const *x, T *const *accin, T ch, T *const *accout,
+                           T *const *uin, T b, T *const *out) {
   RKPass<T> p{};
   for (int k = 0; k < nstate; k++) {
     p.x[k] = x[k];
@@ -292,7 +291,7 @@ void Stepper<T>::stage_pass(int mode, T *const *x, T *const *accin, T ch, T *con
   }
   p.ch = ch;
   p.b = b;
-  rk_pass<T>(prob, mode, nstate, p, st);
+  return rk_pass<T>(prob, mode, nstate, p, st);
 }
 
 template <typename T>
@@ -353,21 +352,23 @@ int Stepper<T>::step(T *const *uin, T *const *uout, T dt, T *const *tape) {
       um = stage_in(0);
       if (ns == 1 && um[0] == uin[0]) copy(acc = utmp, uin);  // smoothed in place below
       copy(um, uin);
-      if (ns == 1) smooth_n(um);
+      if (ns == 1 && (rc = smooth_n(um))) return rc;
       constrain(um);
     }
     for (int m = 0; m < ns - 1; m++) {
       if ((rc = rhs(um, K[0]))) return rc;
       // the tableaux here have one term per stage: beta[m+1][m]
       um = stage_in(m + 1);
-      stage_pass(m == ns - 2 ? RK_MIDS : RK_MID, K[0], acc, (T)cc[m] * h, uacc, uin,
-                 (T)beta[m + 1][m] * h, um);
+      rc = stage_pass(m == ns - 2 ? RK_MIDS : RK_MID, K[0], acc, (T)cc[m] * h, uacc, uin,
+                      (T)beta[m + 1][m] * h, um);
+      if (rc) return rc;
       acc = uacc;
       constrain(um);
       constrain(uacc);
     }
     if ((rc = rhs(um, K[0]))) return rc;
-    stage_pass(RK_LAST, K[0], acc, (T)cc[ns - 1] * h, nullptr, nullptr, T(0), uout);
+    rc = stage_pass(RK_LAST, K[0], acc, (T)cc[ns - 1] * h, nullptr, nullptr, T(0), uout);
+    if (rc) return rc;
     constrain(uout);
     return GF_OK;
   }
@@ -392,8 +393,7 @@ static int ssp_substep(Stepper<T> &S, T *const *u, T *const *x, T dt, T *const *
   int rc = GF_OK;
   if (S.rhs_euler_smooth(u, x, dt, uin, a, y, b, a2, y2, b2, &rc)) return rc;
   if ((rc = S.rhs(u, S.utmp))) return rc;
-  S.euler_smooth_n(S.utmp, x, dt, uin, a, y, b, a2, y2, b2);
-  return GF_OK;
+  return S.euler_smooth_n(S.utmp, x, dt, uin, a, y, b, a2, y2, b2);
 }
 
 // Substep m of the SSP schemes (gexrk_stepper.ipp:533-780): from stage input

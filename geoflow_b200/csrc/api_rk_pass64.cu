@@ -2,16 +2,16 @@
 #include "rk_pass.cuh"
 
 template <>
-void rk_pass<double>(gf_problem *prob, int mode, int nc, const gfk::RKPass<double> &p,
-                 cudaStream_t st) {
+int rk_pass<double>(gf_problem *prob, int mode, int nc, const gfk::RKPass<double> &p,
+                    cudaStream_t st) {
   switch (mode) {
-    case gfk::RK_EULER: gfk::rk_pass_mode<double, gfk::RK_EULER>(prob, nc, p, st); break;
-    case gfk::RK_MID: gfk::rk_pass_mode<double, gfk::RK_MID>(prob, nc, p, st); break;
-    case gfk::RK_MIDS: gfk::rk_pass_mode<double, gfk::RK_MIDS>(prob, nc, p, st); break;
-    case gfk::RK_LAST: gfk::rk_pass_mode<double, gfk::RK_LAST>(prob, nc, p, st); break;
-    case gfk::ADJ_START: gfk::rk_pass_mode<double, gfk::ADJ_START>(prob, nc, p, st); break;
-    case gfk::ADJ_STAGE: gfk::rk_pass_mode<double, gfk::ADJ_STAGE>(prob, nc, p, st); break;
-    case gfk::ADJ_STAGE_LAST: gfk::rk_pass_mode<double, gfk::ADJ_STAGE_LAST>(prob, nc, p, st); break;
-    default: gfk::rk_pass_mode<double, gfk::RK_SMOOTH>(prob, nc, p, st); break;
+    case gfk::RK_EULER: return gfk::rk_pass_mode<double, gfk::RK_EULER>(prob, nc, p, st);
+    case gfk::RK_MID: return gfk::rk_pass_mode<double, gfk::RK_MID>(prob, nc, p, st);
+    case gfk::RK_MIDS: return gfk::rk_pass_mode<double, gfk::RK_MIDS>(prob, nc, p, st);
+    case gfk::RK_LAST: return gfk::rk_pass_mode<double, gfk::RK_LAST>(prob, nc, p, st);
+    case gfk::ADJ_START: return gfk::rk_pass_mode<double, gfk::ADJ_START>(prob, nc, p, st);
+    case gfk::ADJ_STAGE: return gfk::rk_pass_mode<double, gfk::ADJ_STAGE>(prob, nc, p, st);
+    case gfk::ADJ_STAGE_LAST: return gfk::rk_pass_mode<double, gfk::ADJ_STAGE_LAST>(prob, nc, p, st);
+    default: return gfk::rk_pass_mode<double, gfk::RK_SMOOTH>(prob, nc, p, st);
   }
 }

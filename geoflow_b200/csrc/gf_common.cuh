@@ -11,6 +11,7 @@
 
 #include "../../include/gfgpu.h"
 #include "lattice.cuh"
+#include "launch_state.cuh"
 
 #define GF_MAXN 12  // largest GLL point count compiled (p = 11)
 
@@ -185,6 +186,25 @@ inline int dispatch_n(int n, Args &&...args) {
     case 12: return F<12>::run(args...);
     default: return GF_ERR_UNSUPPORTED;
   }
+}
+
+// Raises a kernel's dynamic shared-memory limit on the current device to `bytes`
+// (launch_state.cuh); false when the device refuses it.
+inline bool set_smem_of(const void *kern, size_t bytes) {
+  static gfk::KernelRecord<size_t> limits;
+  int device = 0;
+  cudaGetDevice(&device);
+  return gfk::raise_smem_limit(limits, device, kern, bytes, [&](size_t b) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b) ==
+        cudaSuccess)
+      return true;
+    cudaGetLastError();
+    return false;
+  });
+}
+template <typename K>
+inline bool set_smem(K kern, size_t bytes) {
+  return set_smem_of((const void *)kern, bytes);
 }
 
 inline unsigned grid_for(int64_t n, int threads, int max_blocks) {

@@ -243,9 +243,10 @@ struct RKElemLaunch {
       using E = ElemTile<T, N2>;
       constexpr size_t smem = sizeof(T) * NC * E::CELLS;
       auto kern = k_rk_elem<T, MODE, N2, NC>;
-      static const int resident = [&] {  // blocks per SM
+      if (!set_smem(kern, smem)) return GF_ERR_CUDA;
+      // blocks per SM (of the first device; the same kernel on any sm_100a)
+      static const int resident = [&] {
         int nb = 0;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, EL_THREADS, smem);
         return std::max(nb, 1);
       }();

@@ -2,7 +2,6 @@
 // selected at run time by dispatch_n over the GLL point count.
 #pragma once
 #include <type_traits>
-#include <unordered_map>
 
 #include "gf_common.cuh"
 #include "k_def.cuh"
@@ -16,18 +15,6 @@ namespace gfk {
 
 // Library-wide choice of the FP32 3-d affine apply at p = 7 (gf_set_fp32_apply).
 extern int g_fp32_apply_mode;
-
-// Raises a kernel's dynamic shared-memory limit once per kernel (several
-// kernels share one function type, so the record is keyed by address).
-template <typename K>
-inline void set_smem(K kern, size_t bytes) {
-  static std::unordered_map<const void *, size_t> done;
-  size_t &have = done[(const void *)kern];
-  if (bytes > have) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    have = bytes;
-  }
-}
 
 // Deformed / embedded elements (k_def.cuh): one element per block.
 template <typename T, class LD>

@@ -51,15 +51,15 @@ struct Stepper {
   bool constrains() const;
   void constrain(T *const *u);
   // Smooth on every state component, in place or into out
-  void smooth_n(T *const *v);
-  void smooth_to(T *const *v, T *const *out);
+  int smooth_n(T *const *v);
+  int smooth_to(T *const *v, T *const *out);
   // out = Smooth(the SSP substep update of x = dudt) (y and y2 may be null)
-  void euler_smooth_n(T *const *x, T *const *out, T dt, T *const *uin, T a, T *const *y, T b,
-                      T a2, T *const *y2, T b2);
+  int euler_smooth_n(T *const *x, T *const *out, T dt, T *const *uin, T a, T *const *y, T b,
+                     T a2, T *const *y2, T b2);
   // the class pass after a step_b stage (k_dss.cuh RK_MID, RK_MIDS, RK_LAST):
   // K = Smooth(x), accout = accin + ch K, out = uin + b K or the step's result
-  void stage_pass(int mode, T *const *x, T *const *accin, T ch, T *const *accout, T *const *uin,
-                  T b, T *const *out);
+  int stage_pass(int mode, T *const *x, T *const *accin, T ch, T *const *accout, T *const *uin,
+                 T b, T *const *out);
   // One step uin -> uout.  With a tape (pointers tape[3*m + k], m = 0 ..
   // stages-1), stage m's input state (the argument of its RHS call) is left
   // in tape[3*m + k] for the adjoint sweep.

@@ -4,9 +4,9 @@
 
 #include "k_dss_elem.cuh"
 
-// One pass (RK_* or ADJ_*) on nc state components.
+// One pass (RK_* or ADJ_*) on nc state components; GF_OK or an error code.
 template <typename T>
-void rk_pass(gf_problem *prob, int mode, int nc, const gfk::RKPass<T> &p, cudaStream_t st);
+int rk_pass(gf_problem *prob, int mode, int nc, const gfk::RKPass<T> &p, cudaStream_t st);
 
 namespace gfk {
 
@@ -50,14 +50,12 @@ inline bool elem_pass_ok(const gf_problem *prob, int nc, const RKPass<T> &p) {
 }
 
 template <typename T, int MODE>
-inline void rk_pass_mode(gf_problem *prob, int nc, const RKPass<T> &p, cudaStream_t st) {
+inline int rk_pass_mode(gf_problem *prob, int nc, const RKPass<T> &p, cudaStream_t st) {
   BoxWalk w;
   if (dss_box_walk(prob, w)) {
     if (elem_pass_ok<T, MODE>(prob, nc, p))
-      dispatch_n<RKElemLaunch<T, MODE>::template F>(prob->n, prob, st, nc, p);
-    else
-      dispatch_n<RKBoxLaunch<T, MODE>::template F>(prob->n, prob, st, nc, p);
-    return;
+      return dispatch_n<RKElemLaunch<T, MODE>::template F>(prob->n, prob, st, nc, p);
+    return dispatch_n<RKBoxLaunch<T, MODE>::template F>(prob->n, prob, st, nc, p);
   }
   const SplitCls sc = split_of(prob);
   const int most = prob->ctx->sm_count * 8;
@@ -65,6 +63,7 @@ inline void rk_pass_mode(gf_problem *prob, int nc, const RKPass<T> &p, cudaStrea
   const unsigned nbn = grid_for((sc.n + 3) / 4, 256, most);  // four nodes per thread
   prob->launches += nc;
   for (int j = 0; j < nc; j++) k_rk_split<T, MODE><<<nbs + nbn, 256, 0, st>>>(p, j, sc, nbs);
+  return GF_OK;
 }
 
 }  // namespace gfk
