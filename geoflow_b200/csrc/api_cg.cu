@@ -1535,18 +1535,19 @@ struct Solver {
 
   // small 2-d affine boxes iterate inside one cluster (CL_NODES), whose lines take
   // K1, the operator of a centro-antisymmetric D alone
-  bool cluster_ok() {
-    if (MAP::NPTS == 0 || prob->dim != 2 || !prob->egeom_d || !prob->d_antisym || nL > CL_NODES)
-      return false;
-    if constexpr (MAP::NPTS > 0)
-      if (ctx->cluster_size == 0)
-        ctx->cluster_size = cl_cluster_size(k_cg_cluster<MAP::NPTS>, CL_THREADS);
-    return cl_slab_bytes((int)prob->box.M[0], (int)prob->box.M[1], prob->box.p,
-                         ctx->cluster_size) <= CL_SLAB_MAX;
+  int cluster_size() {  // CTAs, or 0
+    if constexpr (MAP::NPTS > 0) {
+      if (prob->dim != 2 || !prob->egeom_d || !prob->d_antisym || nL > CL_NODES) return 0;
+      const int size = cl_cluster_size(k_cg_cluster<MAP::NPTS>, CL_THREADS, CL_SLAB_MAX);
+      if (size && cl_slab_bytes((int)prob->box.M[0], (int)prob->box.M[1], prob->box.p, size) <=
+                      CL_SLAB_MAX)
+        return size;
+    }
+    return 0;
   }
-  int iterate_cluster(const gf_cg_traits &tr, double p, double q, int use_mass, const double *bL,
-                      double *xL, double *rL, double *w, double *qL, const float *dinv,
-                      double *hist, int *iters) {
+  int iterate_cluster(int size, const gf_cg_traits &tr, double p, double q, int use_mass,
+                      const double *bL, double *xL, double *rL, double *w, double *qL,
+                      const float *dinv, double *hist, int *iters) {
     if constexpr (MAP::NPTS > 0) {
       ClProblem b = cl_problem(prob->box);
       b.egeom = prob->egeom_d;
@@ -1569,12 +1570,9 @@ struct Solver {
       std::copy(prob->W, prob->W + prob->n, B.W);
       b.uniform = prob->egeom_uniform;
       auto kern = k_cg_cluster<MAP::NPTS>;
-      const size_t smem = cl_slab_bytes(b.M0, b.M1, prob->box.p, ctx->cluster_size);
-      set_smem(kern, smem);
-      if (ctx->cluster_size == CL_MAX)
-        GF_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      const size_t smem = cl_slab_bytes(b.M0, b.M1, prob->box.p, size);
       prob->launches++;
-      GF_CUDA(ctx, cl_launch(kern, 1, ctx->cluster_size, CL_THREADS, smem, st, b, B, tr.tol, hist, prob->scal_d));
+      GF_CUDA(ctx, cl_launch(kern, 1, size, CL_THREADS, smem, st, b, B, tr.tol, hist, prob->scal_d));
       GF_CUDA(ctx, cudaMemcpyAsync(prob->scal_h, prob->scal_d, sizeof(double) * S_COUNT,
                                    cudaMemcpyDeviceToHost, st));
       GF_CUDA(ctx, cudaStreamSynchronize(st));
@@ -1697,8 +1695,8 @@ struct Solver {
       double *w = (double *)gf_work(prob, 4, sizeof(double) * nL);
       double *qL = (double *)gf_work(prob, 5, sizeof(double) * nL);
       if (!w || !qL) return gf_fail(ctx, GF_ERR_NOMEM, "CG work allocation failed");
-      if (cluster_ok()) {
-        rc = iterate_cluster(tr, p, q, use_mass, bL, xL, rL, w, qL, d32, hist, &total);
+      if (const int size = cluster_size()) {
+        rc = iterate_cluster(size, tr, p, q, use_mass, bL, xL, rL, w, qL, d32, hist, &total);
       } else {
         rc = residual<double>(p, q, use_mass, bL, xL, qE, rL, rL, w, d32, 0, tr.tol);
         if (rc) return gf_fail(ctx, rc, "residual failed");

@@ -1914,22 +1914,15 @@ extern "C" int gf_ensemble_cg_solve(gf_ensemble_t E, const gf_cg_traits *tr, dou
   // members, the largest of 201 k points: 7.0 ms against 9.4 with the grid-wide
   // iteration, which costs 65-75 us whatever the members.
   size_t slab = 0;
-  const bool cluster = a.fp64 && std::all_of(E->probs.begin(), E->probs.end(),
-                                             [](const gf_problem *m) { return m->d_antisym; });
-  if (cluster) {
-    if (ctx->cluster_size == 0) ctx->cluster_size = cl_cluster_size(k_en_cg_cluster, CL_THREADS);
-    for (int m = 0; m < n; m++) {
-      const EnMember &M = E->host[m];
-      slab = std::max(slab, cl_slab_bytes(M.walk.M[0], M.walk.M[1], M.N - 1, ctx->cluster_size));
-    }
-  }
-  if (cluster && slab <= CL_SLAB_MAX) {
-    GF_CUDA(ctx, cudaFuncSetAttribute(k_en_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)slab));
-    if (ctx->cluster_size == CL_MAX)
-      GF_CUDA(ctx, cudaFuncSetAttribute(k_en_cg_cluster,
-                                        cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    GF_CUDA(ctx, cl_launch(k_en_cg_cluster, n, ctx->cluster_size, CL_THREADS, slab, st, a,
+  int size = 0;
+  if (a.fp64 && std::all_of(E->probs.begin(), E->probs.end(),
+                            [](const gf_problem *m) { return m->d_antisym; }))
+    size = cl_cluster_size(k_en_cg_cluster, CL_THREADS, CL_SLAB_MAX);
+  if (size)
+    for (const EnMember &M : E->host)
+      slab = std::max(slab, cl_slab_bytes(M.walk.M[0], M.walk.M[1], M.N - 1, size));
+  if (size && slab <= CL_SLAB_MAX) {
+    GF_CUDA(ctx, cl_launch(k_en_cg_cluster, n, size, CL_THREADS, slab, st, a,
                            (const int *)E->order_d));
     E->launches++;
   } else if ((rc = en_cg_loop(E, a, S.threads, grid, smem))) {

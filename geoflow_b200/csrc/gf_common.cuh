@@ -22,7 +22,6 @@ struct gf_context {
   int nprob = 0;                // live problems created on this context
   bool destroy_pending = false; // destroyed while problems were alive
   int sm_count = 148;
-  int cluster_size = 0;  // CTAs per cluster of the one-cluster solves; 0: not asked yet
   std::string last_error;
   std::string returned_error;  // storage for gf_ctx_last_error
 };

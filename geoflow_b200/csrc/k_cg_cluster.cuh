@@ -34,7 +34,7 @@
 namespace gfk {
 
 constexpr int CL_THREADS = 512;
-constexpr int CL_MAX = 16;  // CTAs per cluster (non-portable size; 8 elsewhere)
+constexpr int CL_MAX = 16;  // CTAs per cluster (non-portable size; 8 elsewhere, cl_cluster_size)
 
 __device__ __forceinline__ unsigned cl_rank() {
   unsigned r;
@@ -404,24 +404,35 @@ __device__ __forceinline__ void cl_solve_any(const ClProblem &b, ClShared &sh, d
   else cl_solve<N, 0>(b, sh, slab, st, start, hist);
 }
 
-// CTAs per cluster that this kernel can be launched with (16, or the portable 8).
+// CTAs per cluster that this kernel can be launched with, given the most dynamic
+// shared memory that it is ever launched with: 16, the portable 8, or 0 (a device
+// or a partition of one whose GPCs have too few SMs for that memory: the caller
+// then takes the separate kernels).
 template <typename K>
-inline int cl_cluster_size(K kern, int threads) {
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+inline int cl_cluster_size(K kern, int threads, size_t smem) {
+  static KernelRecord<int> sizes;  // of the kernels of this type
+  int device = 0;
+  cudaGetDevice(&device);
+  return cluster_size_for(sizes, device, (const void *)kern, [&](int size) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(CL_MAX);
+    cfg.gridDim = dim3(size);
     cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = CL_MAX;
+    at[0].val.clusterDim.x = size;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0) return CL_MAX;
-  }
-  cudaGetLastError();
-  return 8;
+    const bool ok =
+        set_smem(kern, smem) &&
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, size > 8) ==
+            cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0;
+    cudaGetLastError();
+    return ok;
+  });
 }
 
 template <typename... Exp, typename... Act>

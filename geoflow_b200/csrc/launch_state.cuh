@@ -1,8 +1,9 @@
 // launch_state.cuh -- what the library keeps per kernel between launches: the
-// dynamic shared-memory limit it has raised.  That is an attribute of a kernel ON A
-// DEVICE (another device starts with its own default), and the library is called
-// from several threads, so the record is keyed by (device, kernel) and locked.  Host
-// only, no CUDA calls: the caller passes the call to make.
+// dynamic shared-memory limit it has raised and the cluster size it can be launched
+// with.  Both are attributes of a kernel ON A DEVICE (another device starts with its
+// own defaults), and the library is called from several threads, so the records are
+// keyed by (device, kernel) and locked.  Host only, no CUDA calls: the caller passes
+// the call to make.
 #pragma once
 #include <cstddef>
 #include <map>
@@ -37,6 +38,16 @@ inline bool raise_smem_limit(KernelRecord<size_t> &rec, int device, const void *
     if (!set(bytes)) return false;
     have = bytes;
     return true;
+  });
+}
+
+// CTAs per cluster for (device, kernel): 16 where active(16) says that such a
+// cluster fits, else the portable 8, else 0.  Asked once.
+template <class ACTIVE>
+inline int cluster_size_for(KernelRecord<int> &rec, int device, const void *kernel, ACTIVE active) {
+  return rec.with(device, kernel, [&](int &size) {
+    if (size == 0) size = active(16) ? 16 : (active(8) ? 8 : -1);
+    return size > 0 ? size : 0;
   });
 }
 

@@ -84,16 +84,12 @@ struct RKClusterLaunch {
     static int go(gf_problem *prob, RKProgram<T> &pr, cudaStream_t st) {
       gf_context *ctx = prob->ctx;
       auto kern = k_rk_cluster<T, N, EQN>;
-      if (ctx->cluster_size == 0) ctx->cluster_size = cl_cluster_size(kern, RKC_THREADS);
-      const int size = ctx->cluster_size;
-      if (size == CL_MAX)
-        GF_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
       // elements per group: all CTAs busy, at most 2 N threads per element
       constexpr int most = RKC_THREADS / (2 * N);
+      const int size = cl_cluster_size(kern, RKC_THREADS, sizeof(T) * dudt2_words<N, EQN>() * most);
+      if (!size) return GF_ERR_UNSUPPORTED;
       pr.epb = (int)std::min<int64_t>(most, (prob->ne + size - 1) / size);
       const size_t smem = sizeof(T) * dudt2_words<N, EQN>() * pr.epb;
-      GF_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)(sizeof(T) * dudt2_words<N, EQN>() * most)));
       const Basis<T, N> B = make_basis<T, N>(prob);
       const RunWalk<N - 1> w = RunWalk<N - 1>::make(prob->box);
       prob->launches++;
@@ -105,5 +101,6 @@ struct RKClusterLaunch {
 
 }  // namespace gfk
 
+// GF_ERR_UNSUPPORTED, with nothing launched, on a device that holds no such cluster
 template <typename T>
 int launch_rk_cluster(gf_problem *prob, int eqn, gfk::RKProgram<T> &pr, cudaStream_t st);

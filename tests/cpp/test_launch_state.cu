@@ -68,9 +68,29 @@ static void check_threads() {
       });
 }
 
+static void check_cluster_size() {
+  const int k0 = 0, k1 = 0;
+  for (int largest : {16, 8, 0}) {  // a device that holds clusters of up to so many CTAs
+    KernelRecord<int> rec;
+    int asked = 0;
+    auto active = [&](int size) {
+      asked++;
+      return size <= largest;
+    };
+    CHECK(cluster_size_for(rec, 0, &k0, active) == largest, "largest %d", largest);
+    const int once = asked;
+    CHECK(cluster_size_for(rec, 0, &k0, active) == largest && asked == once, "kept, %d", largest);
+    // a kernel with a need of its own, and another device, are asked for themselves
+    CHECK(cluster_size_for(rec, 0, &k1, [](int size) { return size <= 8; }) == 8, "other kernel");
+    CHECK(cluster_size_for(rec, 1, &k0, [](int) { return false; }) == 0, "other device");
+    CHECK(cluster_size_for(rec, 0, &k0, active) == largest, "unchanged, %d", largest);
+  }
+}
+
 int main() {
   check_smem_limits();
   check_threads();
+  check_cluster_size();
   if (failures) return 1;
   std::printf("launch state ok\n");
   return 0;

@@ -1,6 +1,7 @@
 """What the library keeps per kernel between launches (launch_state.cuh), on the host
 with counted fakes (tests/cpp/test_launch_state.cu): limits belong to a device and a
-kernel, only grow, and are safe with several threads."""
+kernel, only grow, and are safe with several threads; a kernel's cluster size is its
+own, and none where the device holds no such cluster."""
 import shutil
 import subprocess
 from pathlib import Path
