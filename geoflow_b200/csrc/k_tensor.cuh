@@ -122,6 +122,22 @@ __device__ __forceinline__ void node_geom(const Geom<T> &g, int64_t node, NodeGe
 // 2.4 M nodes (N = 7: cap 64, 72, 80, none: 58, 54, 51, 57 us) and 1.7 M (N = 8:
 // 80, 96, 128, none: 58, 50, 43, 49; a cap that spills loses more than the extra
 // warps give; N = 9: 80, 128, none: 74, 59, 104).
+//
+// Two choices by order, each where it measured faster (1.5 M nodes, us; per-node
+// geometry with per-node p and q, with scalar ones, affine with per-node ones):
+// * helm3_regz: the z-column's weights and mass term, which no other thread reads,
+//   stay in registers instead of shared memory (three volumes instead of five)
+//   while they fit there: FP64 N = 2: 18.1 14.4 14.4 against 20.5 18.2 16.4, N = 4:
+//   18.6 12.7 12.4 against 22.6 16.2 15.4, N = 6: 24.5 16.1 14.9 against 28.7 18.5
+//   18.5; from N = 7 it spills (35.2 22.3 22.4 against 30.4 18.5 20.5).  FP32 N = 8:
+//   10.3 10.3 10.3 against 14.4 12.4 13.1; from N = 9 it loses (14.4 12.4 14.4 against
+//   12.4 11.9 12.3).
+// * helm3_joint: the three lines of a thread share one read of a matrix entry
+//   (lines_D).  FP64 from N = 10, where a line at a time spills under the cap (344
+//   bytes at N = 10) and without it leaves two blocks per SM: N = 10: 43 25 27
+//   against 56 39 35 a line at a time and 69 32 39 without a cap; N = 11: 35 21 21
+//   against 44 27 27 and 56 28 31; N = 12: 45 27 27 against 41 25 27 and 90 43 49,
+//   but 10.3 against 12.4 on 17 elements.
 template <typename T, int N> constexpr int epb_diag() {
   return sizeof(T) == 4 ? epb3<N>() : (N <= 2 ? 24 : (96 / (N * N) < 1 ? 1 : 96 / (N * N)));
 }
@@ -129,6 +145,11 @@ template <typename T, int N, int EPB> constexpr int helm3_blocks() {
   constexpr int warps = (N * N * EPB + 31) / 32, regs = N <= 6 ? 56 : (N == 7 ? 80 : 128);
   return sizeof(T) == 4 ? 0 : 65536 / (warps * 32 * regs);
 }
+template <typename T, int N> constexpr bool helm3_regz() {
+  return N <= (sizeof(T) == 4 ? 8 : 6);
+}
+template <typename T, int N> constexpr bool helm3_joint() { return sizeof(T) == 8 && N >= 10; }
+template <typename T, int N> constexpr int helm3_vols() { return helm3_regz<T, N>() ? 3 : 5; }
 template <typename T, int N, int EPB, class LD, typename TO = T>
 __global__ void __launch_bounds__(N *N *EPB, helm3_blocks<T, N, EPB>())
     k_helm3d(const __grid_constant__ Basis<T, N> B, const Geom<T> g, int64_t ne, T p,
@@ -136,9 +157,10 @@ __global__ void __launch_bounds__(N *N *EPB, helm3_blocks<T, N, EPB>())
              const LD ld, TO *__restrict__ uo, const double *__restrict__ stop) {
   if (stop && stop[0] != 0.0) return;
   constexpr int P = Pad<N>::P, PLANE = N * P, VOL = N * PLANE, NN = N * N, NNN = N * N * N;
+  constexpr bool REGZ = helm3_regz<T, N>(), JOINT = helm3_joint<T, N>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *su = reinterpret_cast<T *>(smem_raw) + threadIdx.y * 5 * VOL;
-  T *sx = su + VOL, *sy = su + 2 * VOL, *sz = su + 3 * VOL, *so = su + 4 * VOL;
+  T *su = reinterpret_cast<T *>(smem_raw) + threadIdx.y * helm3_vols<T, N>() * VOL;
+  T *sx = su + VOL, *sy = su + 2 * VOL, *sz = su + 3 * VOL, *so = su + 4 * VOL;  // !REGZ: sz, so
   const int t = threadIdx.x, a0 = t % N, a1 = t / N;
   const int64_t e = (int64_t)blockIdx.x * EPB + threadIdx.y;
   const bool active = e < ne;
@@ -146,6 +168,20 @@ __global__ void __launch_bounds__(N *N *EPB, helm3_blocks<T, N, EPB>())
   const int xl = a1 * PLANE + a0 * P, yl = a1 * PLANE + a0, zl = a1 * P + a0;
 
   // this thread's z-column (i = a0, j = a1): u, the weights, the mass term
+  T rz[REGZ ? N : 1], ro[REGZ ? N : 1];
+  auto put = [&](int k, T u, T wx, T wy, T wz, T o) {
+    const int s = zl + k * PLANE;
+    su[s] = u;
+    sx[s] = wx;
+    sy[s] = wy;
+    if constexpr (REGZ) {
+      rz[k] = wz;
+      ro[k] = o;
+    } else {
+      sz[s] = wz;
+      so[s] = o;
+    }
+  };
   if (active) {
     NodeGeom<T, 3> eg;
     eg.X[0] = eg.X[1] = eg.X[2] = eg.J = T(0);
@@ -156,46 +192,68 @@ __global__ void __launch_bounds__(N *N *EPB, helm3_blocks<T, N, EPB>())
 #pragma unroll
     for (int k = 0; k < N; k++) {
       const int64_t node = base + k * NN + t;
-      const int s = zl + k * PLANE;
       NodeGeom<T, 3> ng = eg;
       node_geom<T, 3>(g, node, ng);
       const T u = (T)lv[k], mass = B.W[k] * w2 * ng.J;
       const T mp = pvec ? mass * pvec[node] : mass * p;
-      su[s] = u;
-      sx[s] = mp * (ng.X[0] * ng.X[0]);
-      sy[s] = mp * (ng.X[1] * ng.X[1]);
-      sz[s] = mp * (ng.X[2] * ng.X[2]);
-      so[s] = use_mass ? mass * (qvec ? qvec[node] : q) * u : T(0);
+      put(k, u, mp * (ng.X[0] * ng.X[0]), mp * (ng.X[1] * ng.X[1]), mp * (ng.X[2] * ng.X[2]),
+          use_mass ? mass * (qvec ? qvec[node] : q) * u : T(0));
     }
   } else {
 #pragma unroll
-    for (int k = 0; k < N; k++) {
-      const int s = zl + k * PLANE;
-      su[s] = sx[s] = sy[s] = sz[s] = so[s] = T(0);
-    }
+    for (int k = 0; k < N; k++) put(k, T(0), T(0), T(0), T(0), T(0));
   }
   __syncthreads();
-  // one line: a = D^T (w (D a))
-  T a[1][N], d[1][N];
-  auto line = [&](const T *w, int s0, int st) {
-#pragma unroll
-    for (int m = 0; m < N; m++) a[0][m] = su[s0 + m * st];
-    lines_D<T, N, 1, false>(B.D, a, [&](int, int i, T v) { d[0][i] = v * w[s0 + i * st]; });
-    lines_D<T, N, 1, true>(B.D, d, [&](int, int i, T v) { a[0][i] = v; });
+  auto wz = [&](int k) -> T {
+    if constexpr (REGZ) return rz[k];
+    else return sz[zl + k * PLANE];
   };
-  line(sx, xl, 1);
+  T oz[N];  // the z-line's D^T (w (D u)); the others' overwrite their weights
+  if constexpr (JOINT) {
+    T a[3][N], d[3][N];
 #pragma unroll
-  for (int m = 0; m < N; m++) sx[xl + m] = a[0][m];
-  line(sy, yl, P);
+    for (int m = 0; m < N; m++) {
+      a[0][m] = su[xl + m];
+      a[1][m] = su[yl + m * P];
+      a[2][m] = su[zl + m * PLANE];
+    }
+    lines_D<T, N, 3, false>(B.D, a, [&](int l, int i, T v) {
+      d[l][i] = v * (l == 0 ? sx[xl + i] : (l == 1 ? sy[yl + i * P] : wz(i)));
+    });
+    lines_D<T, N, 3, true>(B.D, d, [&](int l, int i, T v) {
+      if (l == 0) sx[xl + i] = v;
+      else if (l == 1) sy[yl + i * P] = v;
+      else oz[i] = v;
+    });
+  } else {
+    // one line: a = D^T (w (D a))
+    T a[1][N], d[1][N];
+    auto line = [&](int s0, int st, auto w) {
 #pragma unroll
-  for (int m = 0; m < N; m++) sy[yl + m * P] = a[0][m];
-  line(sz, zl, PLANE);
+      for (int m = 0; m < N; m++) a[0][m] = su[s0 + m * st];
+      lines_D<T, N, 1, false>(B.D, a, [&](int, int i, T v) { d[0][i] = v * w(i); });
+      lines_D<T, N, 1, true>(B.D, d, [&](int, int i, T v) { a[0][i] = v; });
+    };
+    line(xl, 1, [&](int i) { return sx[xl + i]; });
+#pragma unroll
+    for (int m = 0; m < N; m++) sx[xl + m] = a[0][m];
+    line(yl, P, [&](int i) { return sy[yl + i * P]; });
+#pragma unroll
+    for (int m = 0; m < N; m++) sy[yl + m * P] = a[0][m];
+    line(zl, PLANE, wz);
+#pragma unroll
+    for (int m = 0; m < N; m++) oz[m] = a[0][m];
+  }
   __syncthreads();
   if (active) {
 #pragma unroll
     for (int k = 0; k < N; k++) {
       const int s = zl + k * PLANE;
-      uo[base + k * NN + t] = (TO)(((sx[s] + sy[s]) + a[0][k]) + so[s]);
+      const T o = [&] {
+        if constexpr (REGZ) return ro[k];
+        else return so[s];
+      }();
+      uo[base + k * NN + t] = (TO)(((sx[s] + sy[s]) + oz[k]) + o);
     }
   }
 }

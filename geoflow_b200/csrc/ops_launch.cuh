@@ -108,7 +108,7 @@ struct HelmLaunch {
       const Basis<T, N> B = make_basis<T, N>(prob);
       if (prob->dim == 3) {
         constexpr int EPB = epb_diag<T, N>();
-        const size_t smem = sizeof(T) * 5 * N * N * P * EPB;
+        const size_t smem = sizeof(T) * helm3_vols<T, N>() * N * N * P * EPB;
         auto kern = k_helm3d<T, N, EPB, LD, TO>;
         set_smem(kern, smem);
         const unsigned grid = (unsigned)((prob->ne + EPB - 1) / EPB);
