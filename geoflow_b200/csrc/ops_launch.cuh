@@ -117,6 +117,13 @@ struct HelmLaunch {
                                                     uo, stop);
       } else if constexpr (!std::is_same<T, TO>::value) {
         return GF_ERR_UNSUPPORTED;  // mixed storage/arithmetic is 3-d only
+      } else if constexpr (N == 2) {
+        constexpr int EPB = epb2<N>();
+        const size_t smem = sizeof(T) * 3 * N * P * EPB;
+        prob->launches++;
+        k_helm2d_node<T, N, EPB, LD>
+            <<<(unsigned)((prob->ne + EPB - 1) / EPB), dim3(N * N, EPB), smem, st>>>(
+                B, g, prob->ne, p, pvec, q, qvec, use_mass, ld, uo, stop);
       } else {
         constexpr int EPB = epb2l<N>();
         const unsigned grid = (unsigned)((prob->ne + EPB - 1) / EPB);
