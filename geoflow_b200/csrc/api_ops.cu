@@ -302,17 +302,21 @@ struct DssBoxLaunch {
   template <int N>
   struct F {
     static int run(gf_problem *prob, int op, T *u, cudaStream_t st) {
-      const RunWalk<N - 1> w = RunWalk<N - 1>::make(prob->box);
-      const RunGrid g = run_grid(prob, w);
-      prob->launches++;
-      switch (op) {
-        case GF_DSS_SUM: k_dss_box<T, GF_DSS_SUM, N - 1><<<g.blocks, g.block, 0, st>>>(u, w, g); break;
-        case GF_DSS_SMOOTH: k_dss_box<T, GF_DSS_SMOOTH, N - 1><<<g.blocks, g.block, 0, st>>>(u, w, g); break;
-        case GF_DSS_MAX: k_dss_box<T, GF_DSS_MAX, N - 1><<<g.blocks, g.block, 0, st>>>(u, w, g); break;
-        case GF_DSS_MIN: k_dss_box<T, GF_DSS_MIN, N - 1><<<g.blocks, g.block, 0, st>>>(u, w, g); break;
-        default: prob->launches--; return GF_ERR_ARG;
+      if constexpr (N == 2) {
+        return GF_ERR_UNSUPPORTED;  // by points (dss_by_points)
+      } else {
+        const RunWalk<N - 1> w = RunWalk<N - 1>::make(prob->box);
+        const RunGrid g = run_grid(prob, w);
+        prob->launches++;
+        switch (op) {
+          case GF_DSS_SUM: k_dss_box<T, GF_DSS_SUM, N - 1><<<g.blocks, g.block, 0, st>>>(u, w, g); break;
+          case GF_DSS_SMOOTH: k_dss_box<T, GF_DSS_SMOOTH, N - 1><<<g.blocks, g.block, 0, st>>>(u, w, g); break;
+          case GF_DSS_MAX: k_dss_box<T, GF_DSS_MAX, N - 1><<<g.blocks, g.block, 0, st>>>(u, w, g); break;
+          case GF_DSS_MIN: k_dss_box<T, GF_DSS_MIN, N - 1><<<g.blocks, g.block, 0, st>>>(u, w, g); break;
+          default: prob->launches--; return GF_ERR_ARG;
+        }
+        return GF_OK;
       }
-      return GF_OK;
     }
   };
 };
@@ -321,7 +325,7 @@ template <typename T>
 int launch_dss(gf_problem *prob, int op, T *u, cudaStream_t st) {
   BoxWalk w;
   const bool box = dss_box_walk(prob, w);  // lattice classes: no index arrays
-  if (box && w.nL < POINT_NODES) {
+  if (box && dss_by_points(prob, w)) {
     const unsigned grid = grid_for(w.nL, 256, prob->ctx->sm_count * 16);
     prob->launches++;
     switch (op) {

@@ -122,6 +122,21 @@ __device__ __forceinline__ void dss_run(const T *u, const RunWalk<P> &w,
   }
 }
 
+// Whether a gather walks its lattice by points (k_dss_point) or in runs (k_dss_box).
+// Runs save index arithmetic but are p times fewer threads.  They lose where too few
+// are left to cover the latency: lattices of fewer than POINT_NODES points (476 x 476
+// points, p = 7, FP64: 4.9 us, in runs 5.7) and in 3-d, where a run's copies lie
+// further apart, of fewer than RUNS_3D runs (FP64 and FP32 alike: 71^3 points, p = 7,
+// 51 k runs: 6.2 us by points, 8.3 in runs; 73^3, p = 9, 43 k: 6.5 and 8.3; 78^3,
+// p = 11, 43 k: 6.3 and 8.2; even at 78^3, p = 7, 68 k, and 82^3, p = 9, 61 k; runs
+// ahead at 66^3, p = 5, 57 k, FP32, 8.2 and 6.2), and at p = 1, where a run is a point
+// (80^3: FP64 25.5 us by points, 26.7 in runs, FP32 18.5 and 22.3; 549^2: 8.4 and 10.3).
+constexpr int RUNS_3D = 56000;
+inline bool dss_by_points(const gf_problem *prob, const BoxWalk &w) {
+  const int p = prob->n - 1;
+  return p == 1 || w.nL < POINT_NODES || (prob->dim == 3 && w.nL < RUNS_3D * p);
+}
+
 // Box-lattice form of k_dss_split (GGridBox problems, whose classes are the
 // lattice points; no periodic direction with a single element): one thread
 // per run of P lattice points (RunWalk), the members computed from the
@@ -142,8 +157,7 @@ __global__ void __launch_bounds__(256) k_dss_box(T *u, const RunWalk<P> w, const
   w.rest(k, put);
 }
 
-// The same, one thread per point: lattices of fewer than POINT_NODES points
-// (476 x 476 points, p = 7, FP64: 4.9 us, in runs 5.7).
+// The same, one thread per point.
 template <typename T, int OP>
 __global__ void __launch_bounds__(256) k_dss_point(T *__restrict__ u, BoxWalk w) {
   const int stride = gridDim.x * blockDim.x;
