@@ -437,7 +437,7 @@ template <typename T>
 bool Stepper<T>::cluster_ok() const {
   BoxWalk w;
   return prob->dim == 2 && prob->geom <= GF_GEOM_REGULAR && scheme != GF_RK1 &&
-         n * nstate <= RKC_NODES && dss_box_walk(prob, w);
+         rk_cluster_fits(n, nstate, scheme > 4) && dss_box_walk(prob, w);
 }
 
 template <typename T>

@@ -15,9 +15,22 @@
 namespace gfk {
 
 constexpr int RKC_THREADS = 256;
-// Largest grid (element-local nodes times evolved components) that takes the
-// cluster: above it the 148 SMs of the separate kernels win.
-constexpr int64_t RKC_NODES = 40000;
+// Grids that take the cluster: above them the 148 SMs of the separate kernels win.
+// One component is bound by the right-hand side's share of an SM (nodes), more of them
+// also by the class passes (nodes times components).  The crossover moves with the
+// order (whether a CTA's elements fit one group), the scheme, and by a tenth with the
+// host, whose launches the separate kernels wait for (some 5 us each); over 812 grids of
+// p = 1 to 11 these limits leave 0.7 % of time on average against the better side, at
+// most a fifth.  Eight steps in us, cluster against separate kernels (FP64): advection
+// p = 4, RK4, 12.1 k nodes 310, 339, 16.9 k 326, 344, 20.3 k 362, 345; p = 7, 14.4 k
+// 304, 352, 17.4 k 397, 354, 19.6 k 416, 359; Burgers (two components) RK4, p = 5,
+// 9.2 k nodes 369, 394, 13.7 k 471, 423, p = 3, 8.8 k 385, 334, p = 7, 17.4 k 606, 406;
+// SSP33, p = 3, 12.1 k 253, 263, p = 5, 13.7 k 331, 311, p = 9, 14.4 k 305, 362, p = 7,
+// 17.4 k 389, 312; 40 k values, p = 2, SSP33: 480, 214.
+constexpr int64_t RKC_NODES = 18000, RKC_VALUES = 28000, RKC_VALUES_SSP = 30000;
+inline bool rk_cluster_fits(int64_t n, int nstate, bool ssp) {
+  return n <= RKC_NODES && n * nstate <= (ssp ? RKC_VALUES_SSP : RKC_VALUES);
+}
 
 // one stage: the right-hand side of in -> out, then the class pass
 template <typename T>
