@@ -1533,15 +1533,13 @@ struct Solver {
     });
   }
 
-  // small 2-d affine boxes iterate inside one cluster (CL_NODES), whose lines take
+  // small 2-d affine boxes iterate inside one cluster (cl_fits), whose lines take
   // K1, the operator of a centro-antisymmetric D alone
   int cluster_size() {  // CTAs, or 0
     if constexpr (MAP::NPTS > 0) {
-      if (prob->dim != 2 || !prob->egeom_d || !prob->d_antisym || nL > CL_NODES) return 0;
+      if (prob->dim != 2 || !prob->egeom_d || !prob->d_antisym) return 0;
       const int size = cl_cluster_size(k_cg_cluster<MAP::NPTS>, CL_THREADS, CL_SLAB_MAX);
-      if (size && cl_slab_bytes((int)prob->box.M[0], (int)prob->box.M[1], prob->box.p, size) <=
-                      CL_SLAB_MAX)
-        return size;
+      if (size && cl_fits((int)prob->box.M[0], (int)prob->box.M[1], prob->box.p, size)) return size;
     }
     return 0;
   }
