@@ -81,15 +81,17 @@ struct EnMember {
   // box lattice (CG)
   BoxWalk walk;
   int ne0;
-  const uint8_t *maskL8, *multL8;
-  int uniform;
-  double K1[EN_MAXN * EN_MAXN];
+  const uint8_t *maskL8;
   const double *egeom64;
   const float *egeom32;
   const double *bE;
   double *xE, *bL, *xL, *r64, *dinv64, *aE;
   float *dL, *r32, *w32, *q32, *dinv32;
   double *w64, *q64;  // the FP64 solve's search direction and A w
+  // what the cluster solve reads beside these
+  const uint8_t *multL8;
+  int uniform;
+  double K1[EN_MAXN * EN_MAXN];
 };
 
 struct EnCG {
@@ -1910,18 +1912,28 @@ extern "C" int gf_ensemble_cg_solve(gf_ensemble_t E, const gf_cg_traits *tr, dou
   // FP64 members whose direction fits the shared memory of a cluster (about 250 k
   // points) and whose D is centro-antisymmetric (the cluster's lines take K1, which
   // is the operator of no other D): a cluster per member and one launch for the whole
-  // solve.  Twelve
-  // members, the largest of 201 k points: 7.0 ms against 9.4 with the grid-wide
-  // iteration, which costs 65-75 us whatever the members.
+  // solve, unless it would be waiting for the largest member, whose cluster has 16
+  // SMs and whose work goes with its points, halo rows (cl_fits) and N, while the
+  // grid-wide iteration costs 65 us, a little per member and its share of the chip for
+  // all points.  Solves in ms, clusters against grid-wide (elements:p): 48^2:8 5.7, 6.5;
+  // 64^2:7 5.5, 5.4; 56^2:8 7.4, 6.7; 64^2:8 8.9, 6.9; 30x120:7 9.9, 10.9, 120x30:7
+  // 11.5, 10.9; two of 64^2:8 8.9, 8.0, three 10.0, 10.1, six 12.1, 19.6; 64^2:7 and
+  // 63 of 8^2:3 5.7, 6.6, 64^2:8 and those 8.8, 7.9; twelve uneven ones up to 64^2:7
+  // 6.6, 9.3; 64 of 64^2:7 63, 109.
   size_t slab = 0;
   int size = 0;
   if (a.fp64 && std::all_of(E->probs.begin(), E->probs.end(),
                             [](const gf_problem *m) { return m->d_antisym; }))
     size = cl_cluster_size(k_en_cg_cluster, CL_THREADS, CL_SLAB_MAX);
-  if (size)
-    for (const EnMember &M : E->host)
-      slab = std::max(slab, cl_slab_bytes(M.walk.M[0], M.walk.M[1], M.N - 1, size));
-  if (size && slab <= CL_SLAB_MAX) {
+  double wmax = 0.0, wsum = 0.0;
+  for (const EnMember &M : E->host) {
+    if (!size) break;
+    const double w = cl_work(M.walk.M[0], M.walk.M[1], M.N - 1, size) * size * M.N;
+    wmax = std::max(wmax, w);
+    wsum += w;
+    slab = std::max(slab, cl_slab_bytes(M.walk.M[0], M.walk.M[1], M.N - 1, size));
+  }
+  if (size && slab <= CL_SLAB_MAX && wmax <= 1.8e6 + 0.22 * (wsum - wmax) + 4.8e3 * (n - 1)) {
     GF_CUDA(ctx, cl_launch(k_en_cg_cluster, n, size, CL_THREADS, slab, st, a,
                            (const int *)E->order_d));
     E->launches++;
