@@ -316,9 +316,8 @@ bool Stepper<T>::alloc() {
   // the results of all substeps but the last
   const int nK = scheme <= 4 ? 1 : stages() - 1;
   for (int k = 0; k < nstate; k++, slot += 5) {
-    uacc[k] = (T *)gf_work(prob, slot, bytes);
-    utmp[k] = (T *)gf_work(prob, slot + 1, bytes);
-    if (!uacc[k] || !utmp[k]) return false;
+    if (scheme <= 4 && !(uacc[k] = (T *)gf_work(prob, slot, bytes))) return false;
+    if (!(utmp[k] = (T *)gf_work(prob, slot + 1, bytes))) return false;
     for (int j = 0; j < nK; j++)
       if (!(K[j][k] = (T *)gf_work(prob, slot + 2 + j, bytes))) return false;
   }

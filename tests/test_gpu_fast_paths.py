@@ -376,3 +376,23 @@ def test_multigrid_runs(ctx, ne, p):
         assert cg.solve(H, b, x) == 0
         xs.append(x)
     assert rel(*xs) < 1e-8
+
+
+def test_ssp_steps_allocate_what_they_use(ctx):
+    """Work vectors of an SSP advance: one slope and the results of the substeps but
+    the last, per component; none for step_b's running sum."""
+    import torch
+    from geoflow_b200 import GBurgers, GridBox, Problem
+
+    def advance(ne):
+        g = GridBox(3, [ne] * 3, 5)
+        prob = Problem(ctx, g, dirichlet_mask=False)
+        u = prob.zeros(ncomp=3)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        GBurgers(prob, A.GF_EQN_BURGERS, 1e-2, scheme=A.GF_SSP33).step(u, None, dt=1e-4)
+        torch.cuda.synchronize()
+        return (free - torch.cuda.mem_get_info()[0]) / (8 * g.ndof())
+
+    advance(2)  # loads the kernels
+    assert advance(24) < 3 * (1 + 2) + 1  # in vectors of 24 MB
