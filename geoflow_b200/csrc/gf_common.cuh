@@ -190,6 +190,7 @@ inline int dispatch_n(int n, Args &&...args) {
 // Raises a kernel's dynamic shared-memory limit on the current device to `bytes`
 // (launch_state.cuh); false when the device refuses it.
 inline bool set_smem_of(const void *kern, size_t bytes) {
+  if (bytes <= 32 * 1024) return true;  // with its static memory within the default 48 KB
   static gfk::KernelRecord<size_t> limits;
   int device = 0;
   cudaGetDevice(&device);
