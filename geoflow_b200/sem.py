@@ -360,6 +360,12 @@ class _Filter:
         """In place on the state list u (the selected components), or with
         uo given, out of place (u unchanged)."""
         ids = self.istate or list(range(len(u)))
+        # a single field in place of the list would be filtered at each of its nodes
+        # as if a field began there
+        for j in ids:
+            _check_field(self.prob, u[j])
+            if uo is not None:
+                _check_field(self.prob, uo[j])
         if uo is not None:
             for j in ids:
                 uo[j].copy_(u[j])

@@ -80,6 +80,39 @@ def test_filter_matrix_rejects_bad_arguments():
 
 # ------------------------------------------------------------------ GPU ----
 
+def test_filter_refuses_a_field_in_place_of_the_list():
+    """apply takes a list of fields; a single field would be taken for as many fields
+    as it has nodes, each filtered from its node on, past the end of the memory.  On
+    the host, with stand-ins for the tensors."""
+    from types import SimpleNamespace
+    from geoflow_b200 import GBoydFilter, GProjectionFilter
+
+    class Field:
+        is_cuda = True
+
+        def __init__(self, n):
+            self.n = n
+
+        def __len__(self):
+            return self.n
+
+        def __getitem__(self, j):
+            return Field(1)
+
+        def numel(self):
+            return self.n
+
+        def is_contiguous(self):
+            return True
+
+    prob = SimpleNamespace(dim=2, n=4, nlocal=64)
+    for kind in (GBoydFilter, GProjectionFilter):
+        F = kind(prob, 1, 0.1)
+        for u, uo in ((Field(64), None), ([Field(64)], Field(64)), ([Field(48)], None)):
+            with pytest.raises(ValueError, match="N_local"):
+                F.apply(u, None, uo)
+
+
 def dev(a):
     import torch
     return torch.from_numpy(np.ascontiguousarray(a)).to("cuda")
