@@ -237,6 +237,86 @@ def test_solves_with_an_asymmetric_derivative_matrix(ctx, ne, p):
         assert float((r * cuda(g.mask, torch.float64)).abs().max()) < 1e-9 * float(s.abs().max())
 
 
+def stretched(g):
+    """Elements of unequal size: columns and rows of growing width."""
+    eg = g.elem_geom.reshape(g.nelems, 3)
+    e = np.arange(g.nelems)
+    sx, sy = 1.0 + 0.5 * np.sin(e % g.ne[0]), 1.0 + 0.3 * np.cos(e // g.ne[0])
+    eg[:, 0] /= sx
+    eg[:, 1] /= sy
+    eg[:, 2] *= sx * sy
+    return g
+
+
+# more than 2048 points per CTA (16 CTAs), where the vectors are in global memory; rows
+# that do not divide by the CTAs, CTAs without a row; unequal elements; either side
+# of the size limit of the cluster
+@pytest.mark.parametrize("ne,p,per,unequal", [([44, 44], 5, [0, 0], 0), ([50, 35], 6, [1, 0], 1),
+                                              ([3, 700], 4, [0, 1], 0), ([600, 8], 2, [1, 0], 1),
+                                              ([12, 9], 7, [0, 0], 1), ([9, 6], 3, [1, 1], 1),
+                                              ([56, 56], 5, [0, 0], 0), ([57, 57], 5, [0, 0], 0),
+                                              ([160, 16], 5, [0, 0], 0)])
+def test_cluster_cg_large_and_unequal(ctx, ne, p, per, unequal):
+    import torch
+    from geoflow_b200 import CGTraits, GCG, GHelmholtz, GridBox, Problem
+    g = GridBox(2, ne, p, periodic=per)
+    if unequal:
+        g = stretched(g)
+    rng = np.random.default_rng(p)
+    first = g.members[g.class_ptr[:-1]][g.node_class]
+    b = cuda(rng.standard_normal(g.ndof()), torch.float64)
+    x0 = rng.standard_normal(g.ndof())[first]
+    for norm in (A.GF_NORM_EUC, A.GF_NORM_L2):
+        res = []
+        for s in (True, False):
+            prob = Problem(ctx, g, structured=s)
+            H = GHelmholtz(prob)
+            H.set_Lap_scalar(0.02)
+            H.set_mass_scalar(2.0)
+            cg = GCG(CGTraits(maxit=8000, normtype=norm, tol=1e-11, relative=1,
+                              precond=A.GF_PRECOND_JACOBI), prob)
+            x = cuda(x0, torch.float64)
+            assert cg.solve(H, b, prob.zeros(), x) == 0
+            res.append((cg.iter_, x, np.array(cg.get_residuals())))
+        (ia, xa, ha), (ib, xb, hb) = res
+        assert abs(ia - ib) <= max(2, ib // 20)
+        assert rel(xa, xb) < 1e-8
+        assert abs(ha[0] - hb[0]) <= 1e-9 * hb[0]
+
+
+# FP64 ensembles: clusters with members of about 50 k and 200 k points; grid-wide with
+# one member that is too large for the shared memory of a cluster, and with one that
+# the others would wait for; unequal elements and a ragged box on either path
+@pytest.mark.parametrize("boxes", [[([37, 38], 6), ([8, 5], 3), ([64, 64], 7), ([64, 63], 7)],
+                                   [([64, 65], 9), ([9, 14], 8), ([20, 3], 4)],
+                                   [([60, 61], 8), ([7, 5], 6)],
+                                   [([6, 7], 5)]])
+def test_ensemble_fp64_paths_equal_single_solves(ctx, boxes):
+    import torch
+    from geoflow_b200 import CGTraits, Ensemble, GCG, GHelmholtz, GridBox, Problem
+    tr = CGTraits(maxit=8000, normtype=A.GF_NORM_EUC, tol=1e-11, relative=1,
+                  precond=A.GF_PRECOND_JACOBI, precision=A.GF_CG_FP64)
+    grids = [GridBox(2, ne, p) for ne, p in boxes]
+    if len(grids) > 1:
+        grids[1] = stretched(grids[1])
+    rng = np.random.default_rng(len(boxes))
+    bs = [cuda(rng.standard_normal(g.ndof()), torch.float64) for g in grids]
+    probs = [Problem(ctx, g) for g in grids]
+    xs = [p.zeros() for p in probs]
+    rc, it, nrm, st = Ensemble(ctx, probs).solve(bs, xs, tr, p=0.02, q=2.0)
+    assert rc == 0 and list(st) == [0] * len(boxes)
+    for g, b, x, k in zip(grids, bs, xs, it):
+        prob = Problem(ctx, g, structured=False)
+        H = GHelmholtz(prob)
+        H.set_Lap_scalar(0.02)
+        H.set_mass_scalar(2.0)
+        cg = GCG(tr, prob)
+        ref = prob.zeros()
+        assert cg.solve(H, b, prob.zeros(), ref) == 0
+        assert abs(int(k) - cg.iter_) <= max(2, cg.iter_ // 20)
+        assert rel(x, ref) < 1e-8
+
+
 def test_cluster_cg_outcomes(ctx):
     """maxit, an exact start and a non-finite right-hand side."""
     import torch
@@ -331,7 +411,8 @@ def test_reverse_passes_box_equal_csr(ctx, scheme):
 
 
 @pytest.mark.parametrize("ne,p,per", [([33, 31, 33], 2, [0, 1, 0]), ([14, 11, 10], 6, [1, 0, 0]),
-                                      ([7, 8, 9], 9, [1, 1, 0]), ([75, 77], 7, [0, 0]),
+                                      ([7, 8, 9], 9, [1, 1, 0]), ([9, 10, 8], 9, [0, 1, 0]),
+                                      ([40, 41, 43], 1, [1, 0, 0]), ([75, 77], 7, [0, 0]),
                                       ([262, 260], 2, [1, 0])])
 def test_lattice_runs_equal_csr(ctx, ne, p, per):
     """Lattices of more than 2^18 points are walked in runs (smaller ones, point by
