@@ -312,6 +312,13 @@ __device__ __forceinline__ void dudt2d_group(const Basis<T, N> &B, const Geom<T>
   }
 }
 
+// Elements per block: about 256 threads, 128 from N = 9 on, where a block's FP64
+// contractions share one SM for long and a small grid has few blocks (Burgers, FP64,
+// N = 10: 200 elements 8.2 -> 6.2 us, 20 k 108 -> 98; N = 12: 138 elements 10.3 -> 8.2,
+// 13.9 k 115 -> 105; N = 8: 6.2 us either way).
+template <int N> constexpr int epb_dudt2() {
+  return (N >= 9 ? 128 : 256) / (2 * N);
+}
 template <typename T, int N, int EPB, int EQN, int MODE>
 __global__ void __launch_bounds__(2 * N *EPB)
     k_dudt2d(const __grid_constant__ Basis<T, N> B, const Geom<T> g, int64_t ne, T nu,

@@ -197,7 +197,7 @@ inline void launch_dudt_kernel(gf_problem *prob, T nu, const T *const *f, T *con
     kern<<<grid, dim3(N * N, EPB), smem, st>>>(B, g, prob->ne, nu, f[0], f[1], f[2], f[3], imass,
                                                 o[0], o[1], o[2], epi);
   } else {
-    constexpr int EPB = epb2l<N>();
+    constexpr int EPB = epb_dudt2<N>();
     const size_t smem = sizeof(T) * dudt2_words<N, EQN>() * EPB;
     auto kern = k_dudt2d<T, N, EPB, EQN, MODE>;
     set_smem(kern, smem);
