@@ -366,11 +366,11 @@ def dss_timing(ctx, prob, reps=10):
         t = s.elapsed_time(e) / 1e3 / reps
         s_ = 4 if dt == torch.float32 else 8
         # box lattice (k_dss_box): every E-node read and written once, no
-        # index arrays; CSR (k_dss_csr): plus members and class_ptr
+        # index arrays; CSR (k_dss_split): plus members and class_ptr
         box = getattr(prob, "structured", True)
         alg = prob.nlocal * 2 * s_ + (0 if box else prob.nlocal * 4 + prob.grid.nclass * 4)
         out[name] = {"ms": t * 1e3, "alg_bytes": alg, "gbs": alg / t / 1e9,
-                     "kernel": "k_dss_box" if box else "k_dss_csr"}
+                     "kernel": "k_dss_box" if box else "k_dss_split"}
     return out
 
 
@@ -820,6 +820,8 @@ def ensemble_bench(ctx, steps=10, reps=3, members=16, max_level=5, fixed_shape=F
                      "p 3..8), Jacobi PCG to 1e-10 relative EUC residual"),
         "members": [[m[0].ne[0], m[0].p] for m in bm], "n_local_total": nL,
         "tune_s": tune2_s, "shape": E2.shape(),
+        "shape_of": ("the grid-wide iteration of the mixed solves; the FP64 solves of these "
+                     "members take a cluster of blocks each, one launch per solve"),
         "ensemble_s": head["s"], "scheme": head_name,
         "modes": runs,
         "sequential_mixed_s": seqs["mixed"], "sequential_fp64_s": seqs["fp64"],

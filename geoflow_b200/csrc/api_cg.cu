@@ -1881,7 +1881,7 @@ struct MGLevel : MGLevelBase<TM> {
   template <int MODE, bool DOTS>
   void run_pass(TM a1, TM a2, int dsrc, int wd, gf_problem *outer, cudaStream_t st) {
     // FP64 steps, with five vectors of P values a thread, lose more to occupancy than
-    // the runs save: 32^3, p = 7: 127 us a step in runs, 100 by points
+    // the runs save: 32^3, p = 7: 127 us a step in runs, 106 by points
     constexpr bool POINTS = MODE == MG_STEP && sizeof(TM) == 8;
     auto kern = S.map.rw.one ? k_mg_pass_lat<N, MODE, DOTS, TM, true>
                              : k_mg_pass_lat<N, MODE, DOTS, TM, POINTS>;

@@ -1,9 +1,10 @@
 // api_ensemble.cu -- ensembles of independent problems advanced together:
 // one persistent launch per RK stage (2-d deformed and embedded members,
 // e.g. icosahedral-sphere advection cases), or per CG iteration of 2-d box
-// Helmholtz members with FP32 iterations (FP64 residuals and refinement); small
-// members with FP64 iterations take one launch for the whole solve, a cluster of
-// blocks per member (k_cg_cluster.cuh).  The
+// Helmholtz members (FP32 iterations with FP64 residuals and refinement, or FP64
+// iterations).  FP64 iterations take one launch for the whole solve instead, a
+// cluster of blocks per member (k_cg_cluster.cuh), where the members allow it
+// (gf_ensemble_cg_solve).  The
 // reference runs one problem per process; nothing here has a reference
 // counterpart beyond the per-member arithmetic named below.
 //
@@ -30,15 +31,16 @@
 // step_b (rk_stage_point), so each member advances bit for bit as
 // gf_rk_advance advances it alone.  A CG member runs GCG::solve_impl's DFM
 // iteration (solvers/gcg.ipp:239-382) with a Jacobi preconditioner on the
-// unique lattice nodes: FP32 vectors and applies, FP64 dot products, and
-// restarted refinement, x += d and r = mask DSS_Sum(b - A x) in FP64 each
-// time an FP32 run has reduced its residual by inner_tol.  The CG member is
+// unique lattice nodes: in FP64; or with FP32 vectors and applies, FP64 dot
+// products, and restarted refinement, x += d and r = mask DSS_Sum(b - A x) in FP64
+// each time an FP32 run has reduced its residual by inner_tol.  The CG member is
 // the masked (homogeneous Dirichlet) solve, solve_impl (2) with xb = 0: the
 // form without xb leaves bbv_ unset and masks nothing.
 //
 // Tile shapes (threads per block, blocks per SM, team width per order) are
-// chosen by gf_ensemble_tune, which times the element phase of candidate
-// shapes on the ensemble's own data.
+// chosen by gf_ensemble_tune, which times the element phase (RK) or one grid-wide
+// iteration (CG) of candidate shapes on the ensemble's own data; the cluster solve
+// has a shape of its own.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -1042,7 +1044,6 @@ __global__ void __launch_bounds__(CL_THREADS, 1) k_en_cg_cluster(EnArgs a, const
   b.per1 = M.walk.per[1];
   b.M0 = M.walk.M[0];
   b.M1 = M.walk.M[1];
-  b.nL = M.walk.nL;
   b.f0 = M.walk.f0;
   b.egeom = M.egeom64;
   b.mask = M.maskL8;

@@ -101,7 +101,7 @@ __device__ __forceinline__ void cl_total(ClShared &sh, int slot, bool bmax, doub
 
 // One 2-d box problem with affine elements, its vectors on the lattice.
 struct ClProblem {
-  int ne0, ne1, per0, per1, M0, M1, nL;
+  int ne0, ne1, per0, per1, M0, M1;
   FastDiv f0;            // by M0
   const double *egeom;   // dXidX0, dXidX1, Jac per element
   const uint8_t *mask;   // 1 keep, 0 Dirichlet; null: none
@@ -153,7 +153,6 @@ inline ClProblem cl_problem(const BoxLattice &L) {
   c.per1 = L.per[1];
   c.M0 = (int)L.M[0];
   c.M1 = (int)L.M[1];
-  c.nL = c.M0 * c.M1;
   c.f0 = FastDiv::make(c.M0);
   return c;
 }
@@ -446,7 +445,7 @@ inline int cl_cluster_size(K kern, int threads, size_t smem) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, size > 8) ==
             cudaSuccess &&
         cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0;
-    cudaGetLastError();
+    if (!ok) cudaGetLastError();
     return ok;
   });
 }

@@ -170,12 +170,6 @@ __host__ __device__ __forceinline__ int lattice_offsets_qr(int q, int r, int P, 
   o1 = q == ne ? o0 : q * es;
   return q == ne ? 1 : 2;
 }
-template <int P>
-__device__ __forceinline__ int lattice_offsets(int g, int ne, int per, int es, int ls, int &o0,
-                                               int &o1) {
-  const int q = g / P;
-  return lattice_offsets_qr(q, g - q * P, P, ne, per, es, ls, o0, o1);
-}
 
 // The copies of one lattice point: per direction one or two offsets.
 // each() visits them in the (z, y, x) nesting, which is ascending local id

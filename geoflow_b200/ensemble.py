@@ -5,7 +5,8 @@ ones at once on one GPU: one persistent cooperative launch per RK stage of
 every member (deformed / embedded 2-d members, e.g. icosahedral-sphere
 advection) or per CG iteration of every member (2-d box Helmholtz solves:
 FP32 iterations with FP64 residual refinement, or FP64 iterations), captured
-in CUDA graphs.  Small members with FP64 iterations take one launch per solve.
+in CUDA graphs.  FP64 iterations take one launch per solve, a cluster of blocks
+per member, unless a member is too large for that.
 """
 from __future__ import annotations
 
@@ -41,7 +42,9 @@ class Ensemble:
                 scheme=A.GF_RK4):
         """Advances every member's state u[m] in place by nsteps step_b steps
         of dt[m] (a scalar applies to all); c[m] = the member's velocity
-        components (advection)."""
+        components (advection).  One launch per stage serves many small
+        members; for members of more than about half a million nodes a loop
+        of GBurgers.step is faster."""
         n = len(self.problems)
         if len(u) != n:
             raise ValueError(f"{n} states expected")
@@ -76,6 +79,7 @@ class Ensemble:
         return rc, it, nrm, st
 
     # ---- launch shapes ----
+    # (CG: of the grid-wide iteration; a solve with a cluster per member has none)
     def tune(self, dtype=None, reps=5):
         import torch
         code = A.GF_F32 if dtype in (None, torch.float32) else A.GF_F64

@@ -505,8 +505,10 @@ int gf_adjoint_gradient(gf_problem_t prob, const gf_rk_traits *traits,
 /* ---- ensembles of independent problems (no reference counterpart: the
  * reference runs one problem per process) ----
  * Up to 64 2-d members of orders 2..9 advanced together, one persistent
- * cooperative launch per RK stage or CG iteration, captured in CUDA graphs
- * (small members with FP64 iterations: one launch per solve, a cluster each).
+ * cooperative launch per RK stage or CG iteration, captured in CUDA graphs.
+ * CG members with FP64 iterations take one launch per solve instead, a cluster
+ * of thread blocks each, unless one of them is too large for that or its D is not
+ * centro-antisymmetric.
  * Members are either all deformed / embedded problems (GF_ENS_RK: e.g.
  * icosahedral-sphere advection, each member bit-identical to gf_rk_advance
  * on it alone) or all box problems with affine elements (GF_ENS_CG:
@@ -550,7 +552,10 @@ int gf_ensemble_cg_solve(gf_ensemble_t ens, const gf_cg_traits *traits, double p
  * fastest: best of `reps` launches of the RK stage's element phase (on the
  * equation of the last advance; advection before the first) or of one
  * whole CG iteration.  reps < 0 times the current shape |reps| times and
- * changes nothing (its time is then what gf_ensemble_shape reports). */
+ * changes nothing (its time is then what gf_ensemble_shape reports).  For CG
+ * the shape is that of the grid-wide iteration; a solve that takes a cluster per
+ * member (FP64 iterations, see above) launches no such kernel, so neither the
+ * shape nor the tuner's time says anything of it. */
 int gf_ensemble_tune(gf_ensemble_t ens, int dtype, int reps);
 /* The current shape: threads per block, cooperative blocks, lanes per
  * element by GLL point count (team_by_n[n], n <= 10), tuned flag, and the

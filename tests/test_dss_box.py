@@ -1,6 +1,6 @@
-"""Box-lattice gather-scatter (k_dss_box, k_dss_rk_box_n: members computed from
-the lattice point's coordinates) against the CSR kernels (k_dss_csr,
-k_dss_rk_csr: members read from class_ptr/members) on the same grid built
+"""Box-lattice gather-scatter (k_dss_point, k_dss_box, k_rk_box: members computed
+from the lattice point's coordinates) against the CSR kernels (k_dss_split,
+k_rk_split: members read from class_ptr/members) on the same grid built
 without its box description (Problem(structured=False)).  Both fold the
 members of a class in ascending local id (GGFX::doOp, comm/ggfx.hpp:346-443),
 so they agree bit for bit: every op and dtype, with -0.0, NaN and Inf in the
