@@ -130,18 +130,20 @@ inline double cl_work(int M0, int M1, int P, int ctas) {
 }
 // Boxes whose single solve takes the cluster: where it beats the whole chip with a
 // launch per pass.  Beside the lattice points there is a limit on a CTA's work, which
-// a box wide in x reaches early (unless its points stay in
-// registers, cl_solve_any: 400 x 2, p = 5: 27.9, 30.7).  Solves in ms, cluster
-// against separate kernels: squares, 79 k points, p = 3: 0.80, 1.11, p = 5: 1.86,
-// 2.01, p = 7: 3.13, 2.87; 75 k, p = 8: 3.71, 3.45; 68 k, p = 10: 4.96, 4.79; 57 k,
-// p = 7: 2.71, 2.77; 59 k, p = 9: 3.44, 3.79; 64 k, p = 11: 4.68, 5.37.  Wide: 400 x 8
+// a box wide in x reaches early, above all where its halo outweighs its rows (unless
+// its points stay in registers, cl_solve_any: 400 x 2, p = 5: 27.9, 30.7).  Solves in
+// ms, cluster against separate kernels (whose iterations come in batches, so that their
+// time moves by a tenth from box to box): squares, 79 k points, p = 3: 0.80, 1.11,
+// p = 5: 1.86, 2.01, p = 7: 3.13, 2.87; 75 k, p = 8: 3.71, 3.45; 68 k, p = 7: 2.57, 2.96,
+// p = 10: 4.96, 4.79; 59 k, p = 9: 3.44, 3.79; 64 k, p = 11: 4.68, 5.37.  Wide: 400 x 8
 // elements, p = 4 (53 k points): 22.4, 16.6; 700 x 20, p = 2 (57 k): 6.02, 5.35;
-// 160 x 16, p = 5 (65 k): 7.25, 5.50; 60 x 12, p = 8 (47 k): 6.95, 6.74; 40 x 12,
-// p = 8 (31 k): 4.53, 5.81; 300 x 9, p = 3 (25 k): 3.65, 6.55.
+// 160 x 16, p = 5 (65 k): 7.25, 5.50; 60 x 12, p = 8 (47 k): 6.95, 6.74; 150 x 30, p = 4
+// (73 k): 2.25, 2.54; 40 x 12, p = 8 (31 k): 4.53, 5.81; 300 x 9, p = 3 (25 k): 3.65, 6.55.
 inline bool cl_fits(int M0, int M1, int P, int ctas) {
   const int64_t rows = (M1 + ctas - 1) / ctas, nL = (int64_t)M0 * M1;
-  return nL <= (P <= 6 ? 80000 : 64000) &&
-         (M0 * rows <= 4 * CL_THREADS || cl_work(M0, M1, P, ctas) <= 6050.0 * 16 / ctas) &&
+  const double most = (rows >= 2 * P ? 6500.0 : 6050.0) * CL_MAX / ctas;
+  return nL <= (P <= 6 ? 80000 : 68000) &&
+         (M0 * rows <= 4 * CL_THREADS || cl_work(M0, M1, P, ctas) <= most) &&
          cl_slab_bytes(M0, M1, P, ctas) <= CL_SLAB_MAX;
 }
 
